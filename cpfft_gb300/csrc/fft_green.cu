@@ -31,13 +31,41 @@ FftPlan make_plan(int N) {
     p.nst++;
     m /= r;
   };
+  // a prime without a register butterfly comes first (Ns = 1, no twiddles; N <= 256 has at
+  // most one), then as few stages as the radices allow (63 = 7 x 9, 48 = 6 x 8)
+  for (int f = 17; f <= m; f += 2)
+    while (m % f == 0) {
+      bool prime = true;
+      for (int d = 3; d * d <= f; d += 2) prime &= f % d != 0;
+      if (!prime) break;
+      push(f);
+    }
+  for (int r : {13, 11, 7}) while (m % r == 0) push(r);
+  while (m % 9 == 0) push(9);
+  while (m % 5 == 0) push(5);
+  // powers of two, with a left-over 3 folded into a radix 6 where one stage is saved
+  int two = 0;
+  for (int k = m; k % 2 == 0; k /= 2) two++;
+  if (m % 3 == 0 && two % 3 == 1) push(6);
+  while (m % 3 == 0) push(3);
   while (m % 8 == 0) push(8);
   while (m % 4 == 0) push(4);
   while (m % 2 == 0) push(2);
-  for (int f = 3; m > 1; f += 2)
-    while (m % f == 0) push(f);
   return p;
 }
+
+// Threads per block of the shared-memory passes.  A stage has (columns x N / radix)
+// butterflies -- 81 to 162 for the radices 7 to 9 at N = 63 -- so 256 threads leave half of
+// the block idle while its registers (about 112 a thread in FP64) hold back other blocks;
+// below these sizes the grid does not fill the SMs and the wider block shortens the copy
+// loops.  Launches of G(K : x) with 256 / 128 threads, us (ncu, one GB300):
+//   passes A, E  FP64 63: 130 + 93 / 117 + 88; 27: 27 + 18 / 17 + 13; 15: 11.3 + 6.7 / 11.2 + 7.1
+//   pass B       FP64 63: 78 / 75; FP32 40: 9.6 / 8.1; 27: 5.6 / 6.9
+//   pass C       FP64 40: 48 / 38; 27: 26 / 28; FP32 48: 23 / 19; 40: 13.7 / 17.9
+int line_threads(int N) { return N >= 20 ? 128 : 256; }
+int plane_threads(int N) { return N >= 36 ? 128 : 256; }
+template <typename T>
+int column_threads(int N) { return N >= (sizeof(T) == 8 ? 36 : 44) ? 128 : 256; }
 
 template <typename T>
 cudaError_t green_setup(int N) {
@@ -94,13 +122,14 @@ cudaError_t green_apply_dot(const T* x, const T* K4, int flgK, T* y, typename Ve
   // operator's <x, y> is left to the caller on this path
   double* part_a = (g.pre && part && flgK) ? part : nullptr;
   if (part_a && nparts) *nparts = npair * N;
-  pass_a<T, T><<<npair * N, 256, smem_a<T>(N), st>>>(x, K4, flgK, S, g, tw, part_a);
+  const int ta = line_threads(N), tb = plane_threads(N), tc = column_threads<T>(N);
+  pass_a<T, T><<<npair * N, ta, smem_a<T>(N), st>>>(x, K4, flgK, S, g, tw, part_a);
   dim3 gb((H + g.tkb - 1) / g.tkb, N, 9);
-  pass_b<T><<<gb, 256, smem_b<T>(N, g.tkb), st>>>(S, g, tw, 0);
+  pass_b<T><<<gb, tb, smem_b<T>(N, g.tkb), st>>>(S, g, tw, 0);
   dim3 gc((H + g.tkc - 1) / g.tkc, N);
-  pass_c<T><<<gc, 256, smem_c<T>(N, g.tkc), st>>>(S, g, tw);
-  pass_b<T><<<gb, 256, smem_b<T>(N, g.tkb), st>>>(S, g, tw, 1);
-  pass_e<T><<<npair * N, 256, smem_a<T>(N), st>>>(S, y, g, tw);
+  pass_c<T><<<gc, tc, smem_c<T>(N, g.tkc), st>>>(S, g, tw);
+  pass_b<T><<<gb, tb, smem_b<T>(N, g.tkb), st>>>(S, g, tw, 1);
+  pass_e<T><<<npair * N, ta, smem_a<T>(N), st>>>(S, y, g, tw);
   g_kernel_launches += 5;
   return cudaGetLastError();
 }

@@ -57,55 +57,251 @@ __device__ __forceinline__ void dft8(T2* v) {
 }
 
 
-// One forward Stockham stage of radix R on `ncols` columns (column stride cs) from
-// src to dst; tw[k] = exp(-2 pi i k / N).  Radix 2/4/8 run as register butterflies,
-// any other radix evaluates each output as a direct sum (test-only odd sizes).
-template <typename T2, typename T>
-__device__ void stage(const T2* __restrict__ src, T2* __restrict__ dst, int ncols, int cs,
-                      int N, int R, int Ns, const T2* tw) {
-  const int NR = N / R;
-  const int tstride = N / (Ns * R);
-  if (R == 2 || R == 4 || R == 8) {
-    const int total = ncols * NR;
-    for (int t = threadIdx.x; t < total; t += blockDim.x) {
-      int col = t / NR, j = t - col * NR;
-      int jm = j % Ns;
-      int ts = jm * tstride;
-      const T2* s = src + col * cs;
-      T2 v[8];
+// cos and sin of 2 pi j / R, j = 1 .. (R - 1) / 2, of the odd prime radices
+template <int R>
+struct OddRoots;
+template <>
+struct OddRoots<3> {
+  static __device__ __forceinline__ double c(int j) {
+    constexpr double t[] = {-0.5};
+    return t[j];
+  }
+  static __device__ __forceinline__ double s(int j) {
+    constexpr double t[] = {0.866025403784438646763723};
+    return t[j];
+  }
+};
+template <>
+struct OddRoots<5> {
+  static __device__ __forceinline__ double c(int j) {
+    constexpr double t[] = {0.309016994374947424102293, -0.809016994374947424102293};
+    return t[j];
+  }
+  static __device__ __forceinline__ double s(int j) {
+    constexpr double t[] = {0.951056516295153572116439, 0.587785252292473129168706};
+    return t[j];
+  }
+};
+template <>
+struct OddRoots<7> {
+  static __device__ __forceinline__ double c(int j) {
+    constexpr double t[] = {0.623489801858733530525005,
+                                 -0.222520933956314404288903,
+                                 -0.900968867902419126236102};
+    return t[j];
+  }
+  static __device__ __forceinline__ double s(int j) {
+    constexpr double t[] = {0.781831482468029808708445,
+                                 0.974927912181823607018132,
+                                 0.433883739117558120475768};
+    return t[j];
+  }
+};
+template <>
+struct OddRoots<11> {
+  static __device__ __forceinline__ double c(int j) {
+    constexpr double t[] = {0.841253532831181168861812,
+                                 0.415415013001886425529274,
+                                 -0.142314838273285140443793,
+                                 -0.654860733945285064056925,
+                                 -0.959492973614497389890368};
+    return t[j];
+  }
+  static __device__ __forceinline__ double s(int j) {
+    constexpr double t[] = {0.540640817455597582107636,
+                                 0.909631995354518371411715,
+                                 0.989821441880932732376092,
+                                 0.755749574354258283774036,
+                                 0.281732556841429697711418};
+    return t[j];
+  }
+};
+template <>
+struct OddRoots<13> {
+  static __device__ __forceinline__ double c(int j) {
+    constexpr double t[] = {0.885456025653209895900376,
+                                 0.568064746731155802511808,
+                                 0.120536680255323053349068,
+                                 -0.354604887042535625969638,
+                                 -0.748510748171101098634631,
+                                 -0.970941817426052027156982};
+    return t[j];
+  }
+  static __device__ __forceinline__ double s(int j) {
+    constexpr double t[] = {0.464723172043768545656015,
+                                 0.822983865893656394579617,
+                                 0.992708874098053992800752,
+                                 0.935016242685414823439785,
+                                 0.663122658240795202376785,
+                                 0.239315664287557767148754};
+    return t[j];
+  }
+};
+
+// forward DFT of R registers, R an odd prime: the sums and differences of the inputs k and
+// R - k halve the products of the direct form
+template <typename T2, typename T, int R>
+__device__ __forceinline__ void dft_odd(T2* v) {
+  constexpr int h = (R - 1) / 2;
+  T2 a[h], b[h];
+  T2 x0 = v[0];
 #pragma unroll
-      for (int r = 0; r < 8; r++)
-        if (r < R) {
-          T2 x = s[pidx(j + r * NR)];
-          if (r) x = cmul<T2, T>(x, tw[r * ts]);
-          v[r] = x;
-        }
-      if (R == 2) bfly2<T2, T>(v[0], v[1]);
-      else if (R == 4) dft4<T2, T>(v);
-      else dft8<T2, T>(v);
-      T2* d = dst + col * cs;
-      const int base = (j / Ns) * Ns * R + jm;
+  for (int k = 1; k <= h; k++) {
+    a[k - 1].x = v[k].x + v[R - k].x; a[k - 1].y = v[k].y + v[R - k].y;
+    b[k - 1].x = v[k].x - v[R - k].x; b[k - 1].y = v[k].y - v[R - k].y;
+    v[0].x += a[k - 1].x; v[0].y += a[k - 1].y;
+  }
 #pragma unroll
-      for (int r = 0; r < 8; r++)
-        if (r < R) d[pidx(base + r * Ns)] = v[r];
+  for (int m = 1; m <= h; m++) {
+    T2 A = x0, B;
+    B.x = 0; B.y = 0;
+#pragma unroll
+    for (int k = 1; k <= h; k++) {
+      const int j = (k * m) % R, jj = j <= h ? j : R - j;
+      const T c = (T)OddRoots<R>::c(jj - 1), s = (T)(j <= h ? OddRoots<R>::s(jj - 1) : -OddRoots<R>::s(jj - 1));
+      A.x += c * a[k - 1].x; A.y += c * a[k - 1].y;
+      B.x += s * b[k - 1].x; B.y += s * b[k - 1].y;
+    }
+    v[m].x = A.x + B.y; v[m].y = A.y - B.x;
+    v[R - m].x = A.x - B.y; v[R - m].y = A.y + B.x;
+  }
+}
+
+// forward DFT of R registers, natural order in and out
+template <typename T2, typename T, int R>
+__device__ __forceinline__ void dft_regs(T2* v) {
+  if constexpr (R == 2) {
+    bfly2<T2, T>(v[0], v[1]);
+  } else if constexpr (R == 4) {
+    dft4<T2, T>(v);
+  } else if constexpr (R == 8) {
+    dft8<T2, T>(v);
+  } else if constexpr (R == 6) {
+    // 2 x 3 without twiddles (Good-Thomas): input (3 i + 2 j) mod 6, output (3 k + 4 l) mod 6
+    T2 e[3] = {v[0], v[2], v[4]}, o[3] = {v[3], v[5], v[1]};
+    dft_odd<T2, T, 3>(e);
+    dft_odd<T2, T, 3>(o);
+#pragma unroll
+    for (int l = 0; l < 3; l++) bfly2<T2, T>(e[l], o[l]);
+    v[0] = e[0]; v[4] = e[1]; v[2] = e[2];
+    v[3] = o[0]; v[1] = o[1]; v[5] = o[2];
+  } else if constexpr (R == 9) {
+    // 3 x 3: columns of stride 3, twiddles W9^(j k), rows
+    T2 u[3][3];
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      u[j][0] = v[j]; u[j][1] = v[j + 3]; u[j][2] = v[j + 6];
+      dft_odd<T2, T, 3>(u[j]);
+    }
+    constexpr double c9[3] = {0.766044443118978035202393, 0.173648177666930348851717,
+                              -0.939692620785908384054109};  // cos 2 pi {1, 2, 4} / 9
+    constexpr double s9[3] = {0.642787609686539326322643, 0.984807753012208059366743,
+                              0.342020143325668733044099};   // sin 2 pi {1, 2, 4} / 9
+    T2 w1, w2, w4;
+    w1.x = (T)c9[0]; w1.y = (T)-s9[0];
+    w2.x = (T)c9[1]; w2.y = (T)-s9[1];
+    w4.x = (T)c9[2]; w4.y = (T)-s9[2];
+    u[1][1] = cmul<T2, T>(u[1][1], w1);
+    u[1][2] = cmul<T2, T>(u[1][2], w2);
+    u[2][1] = cmul<T2, T>(u[2][1], w2);
+    u[2][2] = cmul<T2, T>(u[2][2], w4);
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      T2 r[3] = {u[0][k], u[1][k], u[2][k]};
+      dft_odd<T2, T, 3>(r);
+      v[k] = r[0]; v[k + 3] = r[1]; v[k + 6] = r[2];
     }
   } else {
-    const int total = ncols * N;
-    const int NoR = N / R;
-    for (int t = threadIdx.x; t < total; t += blockDim.x) {
-      int col = t / N, rem = t - col * N;
-      int j = rem % NR, sidx = rem / NR;  // output s of butterfly j
-      int jm = j % Ns;
-      int ts = jm * tstride;
-      const T2* s = src + col * cs;
-      T2 acc; acc.x = 0; acc.y = 0;
-      for (int r = 0; r < R; r++) {
-        int e = (r * ts + ((r * sidx) % R) * NoR) % N;
-        T2 p = cmul<T2, T>(s[pidx(j + r * NR)], tw[e]);
-        acc.x += p.x; acc.y += p.y;
-      }
-      dst[col * cs + pidx((j / Ns) * Ns * R + jm + sidx * Ns)] = acc;
+    dft_odd<T2, T, R>(v);
+  }
+}
+
+// t / n for 0 <= t < 2^20 and inv = 1 / n (the half keeps the rounding away from integers)
+__device__ __forceinline__ int fdiv(int t, float inv) { return (int)(((float)t + 0.5f) * inv); }
+
+// One forward Stockham stage of radix R on `ncols` columns (column stride cs) from
+// src to dst, one register butterfly a thread; tw[k] = exp(-2 pi i k / N).
+// The FP64 pipe bounds these passes (two FP64 lanes a clock and SM), so the odd radices are
+// register butterflies too: a direct sum takes 4 R FP64 instructions an output, the
+// butterfly of radix 7 about 9, of 9 (as 3 x 3) about 11, and N = 63 needs two stages
+// instead of three.  G(K : x) at 63^3: 1,221 us with direct sums for 3, 5 and 7, 505 us
+// with these stages (FP32: 356 and 91 us); 27^3 129 and 71 us; a prime N, 61^3, 4,800 and
+// 1,740 us (ncu, sum of the five passes).
+template <typename T2, typename T, int R>
+__device__ __forceinline__ void stage_regs(const T2* __restrict__ src, T2* __restrict__ dst,
+                                           int ncols, int cs, int N, int Ns, const T2* tw) {
+  const int NR = N / R, total = ncols * NR;
+  const int tstride = NR / Ns;
+  const float iNR = 1.0f / (float)NR, iNs = 1.0f / (float)Ns;
+  for (int t = threadIdx.x; t < total; t += blockDim.x) {
+    const int col = fdiv(t, iNR), j = t - col * NR;
+    const int jq = fdiv(j, iNs), jm = j - jq * Ns;
+    const T2* s = src + col * cs;
+    T2 v[R];
+#pragma unroll
+    for (int r = 0; r < R; r++) v[r] = s[pidx(j + r * NR)];
+    if (Ns > 1) {
+      const int ts = jm * tstride;
+#pragma unroll
+      for (int r = 1; r < R; r++) v[r] = cmul<T2, T>(v[r], tw[r * ts]);
     }
+    dft_regs<T2, T, R>(v);
+    T2* d = dst + col * cs;
+    const int base = jq * Ns * R + jm;
+#pragma unroll
+    for (int r = 0; r < R; r++) d[pidx(base + r * Ns)] = v[r];
+  }
+}
+
+// The first stage (Ns = 1: no twiddles) for a prime radix without a register butterfly:
+// each thread forms the outputs m and R - m of one butterfly from the sums and differences
+// of the inputs k and R - k.
+template <typename T2, typename T>
+__device__ __forceinline__ void stage_prime(const T2* __restrict__ src, T2* __restrict__ dst,
+                                            int ncols, int cs, int N, int R, const T2* tw) {
+  const int NR = N / R, h = (R - 1) / 2, per = NR * (h + 1), total = ncols * per;
+  const float iper = 1.0f / (float)per, iNR = 1.0f / (float)NR;
+  for (int t = threadIdx.x; t < total; t += blockDim.x) {
+    const int col = fdiv(t, iper), rem = t - col * per;
+    const int m = fdiv(rem, iNR), j = rem - m * NR;
+    const T2* s = src + col * cs;
+    T2* d = dst + col * cs + 0;
+    T2 A = s[pidx(j)], B;
+    B.x = 0; B.y = 0;
+    int e = 0;
+    for (int k = 1; k <= h; k++) {
+      const T2 u = s[pidx(j + k * NR)], w = s[pidx(j + (R - k) * NR)];
+      e += m;
+      if (e >= R) e -= R;
+      const T2 q = tw[e * NR];  // cos, -sin of 2 pi k m / R
+      A.x += q.x * (u.x + w.x); A.y += q.x * (u.y + w.y);
+      B.x -= q.y * (u.x - w.x); B.y -= q.y * (u.y - w.y);
+    }
+    T2 o;
+    o.x = A.x + B.y; o.y = A.y - B.x;
+    d[pidx(j * R + m)] = o;
+    if (m) {
+      o.x = A.x - B.y; o.y = A.y + B.x;
+      d[pidx(j * R + R - m)] = o;
+    }
+  }
+}
+
+template <typename T2, typename T>
+__device__ __forceinline__ void stage(const T2* src, T2* dst, int ncols, int cs, int N, int R,
+                                      int Ns, const T2* tw) {
+  switch (R) {
+    case 2: stage_regs<T2, T, 2>(src, dst, ncols, cs, N, Ns, tw); break;
+    case 3: stage_regs<T2, T, 3>(src, dst, ncols, cs, N, Ns, tw); break;
+    case 4: stage_regs<T2, T, 4>(src, dst, ncols, cs, N, Ns, tw); break;
+    case 5: stage_regs<T2, T, 5>(src, dst, ncols, cs, N, Ns, tw); break;
+    case 6: stage_regs<T2, T, 6>(src, dst, ncols, cs, N, Ns, tw); break;
+    case 7: stage_regs<T2, T, 7>(src, dst, ncols, cs, N, Ns, tw); break;
+    case 8: stage_regs<T2, T, 8>(src, dst, ncols, cs, N, Ns, tw); break;
+    case 9: stage_regs<T2, T, 9>(src, dst, ncols, cs, N, Ns, tw); break;
+    case 11: stage_regs<T2, T, 11>(src, dst, ncols, cs, N, Ns, tw); break;
+    case 13: stage_regs<T2, T, 13>(src, dst, ncols, cs, N, Ns, tw); break;
+    default: stage_prime<T2, T>(src, dst, ncols, cs, N, R, tw); break;  // Ns == 1
   }
 }
 
@@ -128,8 +324,8 @@ __device__ void load_tw(T2* tw_s, const T2* tw_g, int N) {
 
 __device__ __forceinline__ int qmap(int f, int N, int Nhalf, int gmap) {
   if (gmap == CPFFT_G_REF_SHIFT) {
-    int k = ((f - Nhalf) % N + N) % N;
-    return k + 1 - Nhalf;
+    const int k = f - Nhalf;  // 0 <= f < N, 0 < Nhalf <= N
+    return (k < 0 ? k + N : k) + 1 - Nhalf;
   }
   return f <= (N - 1) / 2 ? f : f - N;
 }
@@ -238,6 +434,7 @@ __device__ __forceinline__ dfl kval<dfl, float>(const float* __restrict__ K,
 }
 
 // one partial sum per block of the per-thread values d (fixed order), into *dst
+// (NT: the largest block; blocks may be smaller)
 template <int NT>
 __device__ __forceinline__ void block_partial(double d, double* dst) {
   __shared__ double wsum[NT / 32];
@@ -246,7 +443,7 @@ __device__ __forceinline__ void block_partial(double d, double* dst) {
   __syncthreads();
   if (threadIdx.x == 0) {
     double b = 0.0;
-    for (int k = 0; k < NT / 32; k++) b += wsum[k];
+    for (int k = 0; k < (int)blockDim.x / 32; k++) b += wsum[k];
     *dst = b;
   }
 }
@@ -271,7 +468,7 @@ __global__ void __launch_bounds__(256) pass_a(const T* __restrict__ x, const TK*
   const int bl0 = 2 * bp, bl1 = 2 * bp + 1;
   T dsum = 0;
   for (int t = threadIdx.x; t < 2 * N; t += blockDim.x) {
-    int l = t / N, a = t - l * N;
+    int l = t >= N, a = t - l * N;
     int b = l ? bl1 : bl0;
     T y[9];
     if (b < N) {
@@ -306,9 +503,10 @@ __global__ void __launch_bounds__(256) pass_a(const T* __restrict__ x, const TK*
   __syncthreads();
   T2* r = fft_cols<T2, T>(b0, b1, 9, Lp, g.plan, tw);
   // unpack the two real lines: X0 = (Z + conj Z(-k))/2, X1 = (Z - conj Z(-k))/(2i)
+  const float iH = 1.0f / (float)H;
   for (int t = threadIdx.x; t < 9 * H; t += blockDim.x) {
-    int i = t / H, k = t - i * H;
-    T2 z = r[i * Lp + pidx(k)], w = conjg(r[i * Lp + pidx((N - k) % N)]);
+    int i = fdiv(t, iH), k = t - i * H;
+    T2 z = r[i * Lp + pidx(k)], w = conjg(r[i * Lp + pidx(k ? N - k : 0)]);
     T2 X0, X1;
     X0.x = (T)0.5 * (z.x + w.x); X0.y = (T)0.5 * (z.y + w.y);
     X1.x = (T)0.5 * (z.y - w.y); X1.y = (T)-0.5 * (z.x - w.x);
@@ -333,8 +531,9 @@ __global__ void __launch_bounds__(256) pass_b(typename Vec2<T>::t* __restrict__ 
   const int ka0 = blockIdx.x * TK;
   const int c = blockIdx.y, i = blockIdx.z;
   T2* plane = S + ((long long)i * N + c) * (long long)N * H;
+  const float iTK = 1.0f / (float)TK;
   for (int t = threadIdx.x; t < TK * N; t += blockDim.x) {
-    int row = t / TK, kk = t - row * TK;
+    int row = fdiv(t, iTK), kk = t - row * TK;
     int ka = ka0 + kk;
     T2 v;
     v.x = 0; v.y = 0;
@@ -345,7 +544,7 @@ __global__ void __launch_bounds__(256) pass_b(typename Vec2<T>::t* __restrict__ 
   __syncthreads();
   T2* r = fft_cols<T2, T>(b0, b1, TK, Lp, g.plan, tw);
   for (int t = threadIdx.x; t < TK * N; t += blockDim.x) {
-    int row = t / TK, kk = t - row * TK;
+    int row = fdiv(t, iTK), kk = t - row * TK;
     int ka = ka0 + kk;
     if (ka < H) {
       T2 v = r[kk * Lp + pidx(row)];
@@ -371,10 +570,11 @@ __global__ void __launch_bounds__(256) pass_c(typename Vec2<T>::t* __restrict__ 
   const int ka0 = blockIdx.x * TK;
   const int kb = blockIdx.y;
   const long long cstr = (long long)N * H;  // stride between c planes
+  const float iTK = 1.0f / (float)TK, iN = 1.0f / (float)N;
   // column (i, kk) holds the N values along c
   for (int t = threadIdx.x; t < 9 * N * TK; t += blockDim.x) {
-    int kk = t % TK, rem = t / TK;
-    int c = rem % N, i = rem / N;
+    int rem = fdiv(t, iTK), kk = t - rem * TK;
+    int i = fdiv(rem, iN), c = rem - i * N;
     int ka = ka0 + kk;
     T2 v;
     v.x = 0; v.y = 0;
@@ -388,7 +588,7 @@ __global__ void __launch_bounds__(256) pass_c(typename Vec2<T>::t* __restrict__ 
   const int Nh = g.Nhalf, gm = g.gmap;
   const T scale = (T)g.inv_n3;
   for (int t = threadIdx.x; t < N * TK; t += blockDim.x) {
-    int kc = t / TK, kk = t - kc * TK;
+    int kc = fdiv(t, iTK), kk = t - kc * TK;
     int ka = ka0 + kk;
     T2 A[9], out[9];
 #pragma unroll
@@ -402,8 +602,8 @@ __global__ void __launch_bounds__(256) pass_c(typename Vec2<T>::t* __restrict__ 
                (2 * kc == N || 2 * kb == N || 2 * ka == N);
     if (ka < H && !nyq) {
       int p0 = qmap(kc, N, Nh, gm), p1 = qmap(kb, N, Nh, gm), p2 = qmap(ka, N, Nh, gm);
-      int m0 = qmap((N - kc) % N, N, Nh, gm), m1 = qmap((N - kb) % N, N, Nh, gm),
-          m2 = qmap((N - ka) % N, N, Nh, gm);
+      int m0 = qmap(kc ? N - kc : 0, N, Nh, gm), m1 = qmap(kb ? N - kb : 0, N, Nh, gm),
+          m2 = qmap(ka ? N - ka : 0, N, Nh, gm);
       if (m0 == -p0 && m1 == -p1 && m2 == -p2) {
         green_acc<T2, T>(g.pre, s_coef, A, p0, p1, p2, scale, out);
       } else {
@@ -421,8 +621,8 @@ __global__ void __launch_bounds__(256) pass_c(typename Vec2<T>::t* __restrict__ 
   __syncthreads();
   T2* r2 = fft_cols<T2, T>(o, r, 9 * TK, Lp, g.plan, tw);
   for (int t = threadIdx.x; t < 9 * N * TK; t += blockDim.x) {
-    int kk = t % TK, rem = t / TK;
-    int c = rem % N, i = rem / N;
+    int rem = fdiv(t, iTK), kk = t - rem * TK;
+    int i = fdiv(rem, iN), c = rem - i * N;
     int ka = ka0 + kk;
     if (ka < H) {
       T2 v = r2[(i * TK + kk) * Lp + pidx(c)];
@@ -449,8 +649,9 @@ __global__ void __launch_bounds__(256) pass_e(const typename Vec2<T>::t* __restr
   const int bp = blockIdx.x % npair, c = blockIdx.x / npair;
   const int bl0 = 2 * bp, bl1 = 2 * bp + 1;
   const bool even = (N % 2) == 0;
+  const float iN = 1.0f / (float)N, i9N = 1.0f / (float)(9 * N);
   for (int t = threadIdx.x; t < 9 * N; t += blockDim.x) {
-    int i = t / N, k = t - i * N;
+    int i = fdiv(t, iN), k = t - i * N;
     long long base = ((long long)i * N + c) * N;
     int kk = k < H ? k : N - k;
     T2 X0 = S[(base + bl0) * H + kk], X1;
@@ -467,8 +668,8 @@ __global__ void __launch_bounds__(256) pass_e(const typename Vec2<T>::t* __restr
   __syncthreads();
   T2* r = fft_cols<T2, T>(b0, b1, 9, Lp, g.plan, tw);
   for (int t = threadIdx.x; t < 2 * 9 * N; t += blockDim.x) {
-    int l = t / (9 * N), rem = t - l * 9 * N;
-    int i = rem / N, a = rem - i * N;
+    int l = fdiv(t, i9N), rem = t - l * 9 * N;
+    int i = fdiv(rem, iN), a = rem - i * N;
     int b = l ? bl1 : bl0;
     if (b < N) {
       T2 z = r[i * Lp + pidx(a)];  // conj of the unscaled inverse
