@@ -16,7 +16,10 @@
 // The reference's result is Re(IDFT(Ghat(q(f)) X(f))); for real input that equals
 // IDFT(Hs(f) X(f)) with Hs(f) = (Ghat(q(f)) + Ghat(q(-f)))/2, which keeps the half
 // spectrum Hermitian and is what pass C applies, for both frequency mappings.
+#include <algorithm>
+
 #include "green_passes.cuh"
+#include "green_small.cuh"
 
 
 FftPlan make_plan(int N) {
@@ -67,6 +70,91 @@ int plane_threads(int N) { return N >= 36 ? 128 : 256; }
 template <typename T>
 int column_threads(int N) { return N >= (sizeof(T) == 8 ? 36 : 44) ? 128 : 256; }
 
+// ---- small grids: planes forward, columns, planes inverse (green_small.cuh) -------------
+template <typename T, bool SPLIT>
+__global__ void __launch_bounds__(256) small_forward(const T* __restrict__ x, const T* __restrict__ K4,
+                                                     int flgK, typename Vec2<T>::t* __restrict__ S,
+                                                     GridDesc g, const typename Vec2<T>::t* __restrict__ twg,
+                                                     double* __restrict__ part) {
+  using T2 = typename Vec2<T>::t;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int N = g.N;
+  const long long N3 = g.N3;
+  T2* tw = reinterpret_cast<T2*>(smem_raw);
+  T2* b0 = tw + N;
+  load_tw(tw, twg, N);
+  const int i = blockIdx.x / N, c0 = blockIdx.x - i * N;
+  const long long v0 = (long long)N * N * c0;
+  T dsum = 0;
+  plane_forward<T2, T, SPLIT>(
+      [&](int u) {
+        const long long v = v0 + u;
+        if (!flgK) return x[i * N3 + v];
+        T xv[9], s = 0;
+#pragma unroll
+        for (int j = 0; j < 9; j++) xv[j] = x[j * N3 + v];
+#pragma unroll
+        for (int j = 0; j < 9; j++) s += K4[(9 * i + j) * N3 + v] * xv[j];
+        if (part) dsum += s * x[i * N3 + v];
+        return s;
+      },
+      S, i, c0, g, tw, b0, b0 + std::max(plane_cols(N), 3 * SMALL_TKC) * padlen(N));
+  if (part) block_partial<256>((double)dsum, part + blockIdx.x);
+}
+
+template <bool SPLIT>
+__global__ void __launch_bounds__(128) small_columns(double2* __restrict__ S, GridDesc g,
+                                                     const double2* __restrict__ twg) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  double2* tw = reinterpret_cast<double2*>(smem_raw);
+  double2* b0 = tw + g.N;
+  load_tw(tw, twg, g.N);
+  column_tile<double2, double, SPLIT>(S, blockIdx.z, blockIdx.y, blockIdx.x * SMALL_TKC, g, tw, b0,
+                                      b0 + 3 * SMALL_TKC * padlen(g.N));
+}
+
+template <typename T, bool SPLIT>
+__global__ void __launch_bounds__(256) small_inverse(const typename Vec2<T>::t* __restrict__ S,
+                                                     T* __restrict__ y, GridDesc g,
+                                                     const typename Vec2<T>::t* __restrict__ twg) {
+  using T2 = typename Vec2<T>::t;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int N = g.N;
+  T2* tw = reinterpret_cast<T2*>(smem_raw);
+  T2* b0 = tw + N;
+  load_tw(tw, twg, N);
+  const int i = blockIdx.x / N, c0 = blockIdx.x - i * N;
+  T* out = y + i * g.N3 + (long long)N * N * c0;
+  plane_inverse<T2, T, SPLIT>([&](int u, T v) { out[u] = v; }, S, i, c0, g, tw, b0,
+                              b0 + std::max(plane_cols(N), 3 * SMALL_TKC) * padlen(N));
+}
+
+// The largest grid of the three-pass form.  It saves two launches and one round trip of the
+// half spectrum and balances better, but a plane tile reads all nine components of x for
+// each one it writes and its FP64 stages fill the lanes less well than the wider line and
+// column tiles.  Three against five passes, us per G(K : x) (ncu, one GB300): FP64 9^3 24 / 61,
+// 16^3 36 / 46, 24^3 51 / 58, 32^3 69 / 95 (register passes), 48^3 204 / 212, 56^3 367 / 331;
+// FP32 15^3 21 / 31, 27^3 30 / 37, 48^3 47 / 59, 63^3 75 / 90, 80^3 174 / 193, 96^3 306 / 309.
+template <typename T>
+constexpr int small_max() { return sizeof(T) == 8 ? 48 : 80; }
+
+template <typename T, bool SPLIT>
+void small_apply(const T* x, const T* K4, int flgK, T* y, typename Vec2<T>::t* S,
+                 const typename Vec2<T>::t* tw, const GridDesc& g, cudaStream_t st, double* part) {
+  const int N = g.N;
+  const size_t sm = smem_small<T>(N);
+  constexpr int BT = 256;
+  small_forward<T, SPLIT><<<9 * N, BT, sm, st>>>(x, K4, flgK, S, g, tw, part);
+  if constexpr (sizeof(T) == 8) {
+    small_columns<SPLIT><<<dim3((g.H + SMALL_TKC - 1) / SMALL_TKC, N, 3), 128, sm, st>>>(S, g, tw);
+  } else {
+    GridDesc gc = g;
+    gc.tkc = tile_c<T>();
+    pass_c<T><<<dim3((g.H + gc.tkc - 1) / gc.tkc, N), column_threads<T>(N), smem_c<T>(N, gc.tkc), st>>>(S, gc, tw);
+  }
+  small_inverse<T, SPLIT><<<9 * N, BT, sm, st>>>(S, y, g, tw);
+}
+
 template <typename T>
 cudaError_t green_setup(int N) {
   cudaError_t e;
@@ -74,7 +162,9 @@ cudaError_t green_setup(int N) {
   // the shared-memory Stockham passes at 128^3, measured on a GB300)
   {
     switch (N) {
-      case 32: return wgreen_setup<1, T>();
+      case 32:
+        if constexpr (sizeof(T) == 4) return wgreen_setup<1, T>();
+        break;
       case 64: return wgreen_setup<2, T>();
       case 128: return wgreen_setup<4, T>();
       case 256: return wgreen_setup<8, T>();
@@ -88,6 +178,12 @@ cudaError_t green_setup(int N) {
   if ((e = raise_max_dynamic_smem((const void*)pass_b<T>, b))) return e;
   if ((e = raise_max_dynamic_smem((const void*)pass_c<T>, c))) return e;
   if ((e = raise_max_dynamic_smem((const void*)pass_e<T>, a))) return e;
+  {
+    const size_t sm = smem_small<T>(N);
+    if ((e = raise_max_dynamic_smem((const void*)small_forward<T, false>, sm))) return e;
+    if ((e = raise_max_dynamic_smem((const void*)small_inverse<T, false>, sm))) return e;
+    if ((e = raise_max_dynamic_smem((const void*)small_columns<false>, smem_small<double>(N)))) return e;
+  }
   return cudaSuccess;
 }
 
@@ -102,7 +198,12 @@ cudaError_t green_apply_dot(const T* x, const T* K4, int flgK, T* y, typename Ve
   {
     warp_path = true;
     switch (N) {
-      case 32: wgreen_apply<1, T>(x, K4, nullptr, flgK, y, S, tw, g, st, part, rfuse, scf); break;
+      case 32:
+        if constexpr (sizeof(T) == 4)
+          wgreen_apply<1, T>(x, K4, nullptr, flgK, y, S, tw, g, st, part, rfuse, scf);
+        else
+          warp_path = false;
+        break;
       case 64: wgreen_apply<2, T>(x, K4, nullptr, flgK, y, S, tw, g, st, part, rfuse, scf); break;
       case 128: wgreen_apply<4, T>(x, K4, nullptr, flgK, y, S, tw, g, st, part, rfuse, scf); break;
       case 256: wgreen_apply<8, T>(x, K4, nullptr, flgK, y, S, tw, g, st, part, rfuse, scf); break;
@@ -110,6 +211,22 @@ cudaError_t green_apply_dot(const T* x, const T* K4, int flgK, T* y, typename Ve
     }
   }
   if (rfuse && !warp_path) return cudaErrorNotSupported;  // the fused update needs the warp passes
+  if (N <= small_max<T>() && !warp_path) {
+    double* part_a = (g.pre && part && flgK) ? part : nullptr;
+    if (part_a && nparts) *nparts = 9 * N;
+    if constexpr (sizeof(T) == 8) {
+      if (N <= 16) {  // split stages: 15^3 33 against 38 us, 20^3 63 against 42
+        g.plan = split_plan(N);
+        small_apply<T, true>(x, K4, flgK, y, S, tw, g, st, part_a);
+      } else {
+        small_apply<T, false>(x, K4, flgK, y, S, tw, g, st, part_a);
+      }
+    } else {
+      small_apply<T, false>(x, K4, flgK, y, S, tw, g, st, part_a);
+    }
+    g_kernel_launches += 3;
+    return cudaGetLastError();
+  }
   if (warp_path) {
     if (part && nparts) *nparts = (N / 2) * N;
     g_kernel_launches += 5;

@@ -24,8 +24,9 @@ def green_ref(x, N, centered):
 
 
 # first stages of 2..13, a prime above 13 alone and with 2 and 3, squares, 2- and 3-stage
-# plans on both sides of every block-size rule (20, 36, 44)
-SIZES = [2, 3, 6, 7, 9, 11, 13, 17, 18, 19, 22, 26, 33, 34, 35, 36, 39, 43, 45, 49, 51, 61, 63, 66]
+# plans on both sides of every rule (split stages 16, three passes 48 and 80, blocks 20, 36, 44)
+SIZES = [2, 3, 6, 7, 9, 11, 13, 16, 17, 18, 19, 22, 26, 33, 34, 35, 36, 39, 43, 45, 48, 49, 51, 61,
+         63, 66, 80, 81]
 
 
 @pytest.mark.gpu
