@@ -35,6 +35,7 @@ cudaError_t f2disp_device(const double* F, int N, double lx, double ly, double l
 bool mlp_device_weights(mlp::Weights* w, int** err);
 int mlp_check_error();
 #include "krylov.cuh"
+#include "cg_small.cuh"
 
 // per host thread: a thread drives one context (cpfft_batch_solve runs several at once)
 static thread_local char g_err[512] = "";
@@ -448,6 +449,7 @@ struct Ctx {
   double2* tw = nullptr;
   float2* twf = nullptr;
   double *part = nullptr, *sc = nullptr, *h_sc = nullptr;
+  unsigned* bar = nullptr;  // grid-barrier counter of the one-launch CG (cg_small.cu)
   unsigned long long* stats = nullptr;
   unsigned long long* h_stats = nullptr;
   bool K4f_valid = false;
@@ -552,7 +554,7 @@ void free_ctx(Ctx* c) {
                   c->hist[0], c->hist[1], c->K4f, c->xf, c->rf, c->pf, c->Apf, c->ori, c->crys,
                   c->oris, c->cryss, c->S, c->Sf, c->tw, c->twf, c->part, c->sc, c->stats,
                   c->k0sum, c->K4lo, c->twdf, c->vcost, c->vperm, c->vq, c->pre_dev,
-                  c->mises, c->misess};
+                  c->mises, c->misess, c->bar};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (c->h_sc) cudaFreeHost(c->h_sc);
@@ -761,9 +763,39 @@ int matvec32_pre(Ctx* c, const float* x, float* y, int flgK, bool want_alpha) {
   return 0;
 }
 
+// cg64 on a small grid: the whole solve in one launch (cg_small.cu), one host wait
+int cg64_small(Ctx* c, const double* b, double* x, double tol, int* iters) {
+  const int maxIter = 1000;
+  *iters = 0;
+  if (!(tol > 2.220446049250313e-16 && tol < 1.0)) return CPFFT_ERR_CG_TOL;
+  kt_start(c, KT_G64);
+  CK(cg_small_solve(b, x, c->r, c->p, c->w, c->Ap, c->K4, c->S, c->tw, c->g, tol, maxIter, c->part,
+                    c->sc, c->bar, c->st));
+  TRY(kt_stop(c));
+  CK(cudaMemcpyAsync(c->h_sc, c->sc, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  TRY(sync(c));
+  const int stop = (int)c->h_sc[SC_STOP], it = (int)c->h_sc[SC_CNT];
+  if (stop == STOP_BARRIER) {
+    cpfft_set_error("CG: a grid barrier ran out of its wait");
+    return CPFFT_ERR_CUDA;
+  }
+  if (stop == STOP_NONFINITE) {
+    *iters = it;
+    cpfft_set_error(it ? "CG residual is not finite" : "non-finite CG right-hand side");
+    return CPFFT_ERR_NONFINITE;
+  }
+  *iters = it;
+  if (!it) return 0;  // ||b|| at round-off: x = 0
+  c->f64_matvecs += it;
+  c->cg_iters += it;
+  c->cg_solves++;
+  return stop == STOP_MAXIT ? CPFFT_ERR_CG_MAXIT : 0;
+}
+
 // fftPcg (src/FFT_nr3.f:214-360), plain FP64: CG from x = 0 with the stop test
 // ||r|| <= tol*||b|| .or. ||r|| <= tol and at most 1000 iterations
 int cg64(Ctx* c, const double* b, double* x, double tol, int* iters) {
+  if (cg_small_fp64(c->N)) return cg64_small(c, b, x, tol, iters);
   const long long n = 9 * c->N3;
   const int maxIter = 1000;
   *iters = 0;
@@ -1692,7 +1724,7 @@ int cpfft_init(int N, const int* matList, const double* kocks_deg, const cpfft_c
       (rc = dalloc(c->cryss, ncrystals * sizeof(CrysRec))) ||
       (rc = dalloc(c->S, (size_t)9 * N * N * c->g.H * sizeof(double2))) ||
       (rc = dalloc(c->tw, N * sizeof(double2))) || (rc = dalloc(c->part, (size_t)std::max<long long>(9 * NPART, (long long)N * N) * sizeof(double))) ||
-      (rc = dalloc(c->sc, SC_COUNT * sizeof(double))) ||
+      (rc = dalloc(c->sc, SC_COUNT * sizeof(double))) || (rc = dalloc(c->bar, sizeof(unsigned))) ||
       (rc = dalloc(c->stats, 8 * sizeof(unsigned long long))))
     return fail(rc);
   if (cudaMallocHost((void**)&c->h_sc, SC_COUNT * sizeof(double)) != cudaSuccess ||
@@ -2510,7 +2542,7 @@ int cpfft_nr3_step(int step, const double* BC, const int* isNBC, double tolNR, d
   S.t_stress_kernel = c->kt_acc[KT_STRESS];
   S.t_green64 = c->kt_acc[KT_G64];
   S.t_green32 = c->kt_acc[KT_G32];
-  S.n_green64 = c->kt_cnt[KT_G64];
+  S.n_green64 = c->f64_matvecs;
   S.n_green32 = c->f32_matvecs;
   S.n_green32_timed = c->kt_cnt[KT_G32];
   S.t_cg_graph = c->kt_acc[KT_CGGRAPH];

@@ -17,7 +17,7 @@ enum {
   SC_COUNT = 32
 };
 // SC_STOP values
-enum { STOP_NONE = 0, STOP_TEST = 1, STOP_MAXIT = 2, STOP_NONFINITE = 3 };
+enum { STOP_NONE = 0, STOP_TEST = 1, STOP_MAXIT = 2, STOP_NONFINITE = 3, STOP_BARRIER = 4 };
 enum { OP_STORE = 0, OP_ALPHA = 1, OP_BETA = 2 };
 
 cudaError_t dev_dot(const double* a, const double* b, long long n, double* part, double* sc,

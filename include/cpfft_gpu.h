@@ -147,7 +147,8 @@ typedef struct cpfft_stats {
     double    t_total;          /* seconds in the whole call (host clock)                  */
     double    t_device;         /* seconds between CUDA events at the call's start and end */
     double    t_stress_kernel;  /* summed CUDA-event time of the stress-update kernel      */
-    double    t_green64;        /* summed CUDA-event time of FP64-accurate Green applies   */
+    double    t_green64;        /* summed CUDA-event time of FP64-accurate Green applies (on
+                                   grids up to 33^3 of the plain FP64 CG's whole solves)   */
     double    t_green32;        /* summed CUDA-event time of the timed FP32 Green applies  */
     long long n_green64;        /* FP64-accurate Green applies (FP64 or double-float)      */
     long long n_green32;        /* FP32 Green applies                                      */
