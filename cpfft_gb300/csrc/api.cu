@@ -341,6 +341,24 @@ void mrr_interaction(int slip_type, double Gm[144], double Hm[144]) {
     }
 }
 
+// the table of x^y (PowTab); entries rounded once from long double
+bool pow_table(double y, PowTab& t) {
+  if (!(y > 0.0 && y <= 8.0)) return false;
+  t.y = y;
+  long double b = 1.0L;
+  for (int k = 1; k <= 6; k++) {
+    b *= ((long double)y - (k - 1)) / k;
+    t.c[k - 1] = (double)b;
+  }
+  for (int i = 0; i < PowTab::NM; i++) {
+    t.rc[i] = (double)(1.0L / (1.0L + (i + 0.5L) / PowTab::NM));
+    t.P[i] = (double)powl((long double)t.rc[i], -(long double)y);
+  }
+  // 2^(y k), infinite or zero past the exponent range as x^y is
+  for (int k = 0; k < PowTab::NE; k++) t.E[k] = (double)exp2l((long double)y * (k - PowTab::EMID));
+  return true;
+}
+
 CrysRec crystal_record(const cpfft_crystal& p) {
   CrysRec c;
   std::memset(&c, 0, sizeof(c));
@@ -436,6 +454,7 @@ struct Ctx {
   int *ori = nullptr, *crys = nullptr;
   OriRec* oris = nullptr;
   CrysRec* cryss = nullptr;
+  PowTab* ptabs = nullptr;  // the crystals' power tables
   // materials: 0-based material of every voxel; per material 0 = crystal, 1 = mm01
   // (cpfft_set_mises), 2 = declared non-crystal and not yet defined
   std::vector<int> mat;
@@ -554,7 +573,7 @@ void free_ctx(Ctx* c) {
                   c->hist[0], c->hist[1], c->K4f, c->xf, c->rf, c->pf, c->Apf, c->ori, c->crys,
                   c->oris, c->cryss, c->S, c->Sf, c->tw, c->twf, c->part, c->sc, c->stats,
                   c->k0sum, c->K4lo, c->twdf, c->vcost, c->vperm, c->vq, c->pre_dev,
-                  c->mises, c->misess, c->bar};
+                  c->mises, c->misess, c->bar, c->ptabs};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (c->h_sc) cudaFreeHost(c->h_sc);
@@ -1629,6 +1648,18 @@ int cpfft_init(int N, const int* matList, const double* kocks_deg, const cpfft_c
     h_type = p.h_type;
     cr[k] = crystal_record(p);
   }
+  // power tables of the crystals whose exponents need them
+  std::vector<PowTab> tabs;
+  std::vector<int> tab_n1(ncrystals, -1), tab_c8(ncrystals, -1);
+  for (int k = 0; k < ncrystals; k++) {
+    if (props[k].slip_type == CPFFT_NOT_A_CRYSTAL) continue;
+    PowTab t;
+    if ((h_type == 7 || h_type == 4) ? pow_table(props[k].tau_hat_v, t)
+                                     : cr[k].n_int < 0 && pow_table(props[k].harden_n - 1.0, t)) {
+      ((h_type == 7 || h_type == 4) ? tab_c8 : tab_n1)[k] = (int)tabs.size();
+      tabs.push_back(t);
+    }
+  }
   if (first_crystal >= 0) slip_geometry(props[first_crystal].slip_type, bb, nn);
   if (!nslip) nslip = 12;
   // distinct (crystal, orientation) records; a voxel of another material points at the
@@ -1722,6 +1753,7 @@ int cpfft_init(int N, const int* matList, const double* kocks_deg, const cpfft_c
       (rc = dalloc(c->ori, N3 * sizeof(int))) || (rc = dalloc(c->crys, N3 * sizeof(int))) ||
       (rc = dalloc(c->oris, oris.size() * sizeof(OriRec))) ||
       (rc = dalloc(c->cryss, ncrystals * sizeof(CrysRec))) ||
+      (tabs.size() && (rc = dalloc(c->ptabs, tabs.size() * sizeof(PowTab)))) ||
       (rc = dalloc(c->S, (size_t)9 * N * N * c->g.H * sizeof(double2))) ||
       (rc = dalloc(c->tw, N * sizeof(double2))) || (rc = dalloc(c->part, (size_t)std::max<long long>(9 * NPART, (long long)N * N) * sizeof(double))) ||
       (rc = dalloc(c->sc, SC_COUNT * sizeof(double))) || (rc = dalloc(c->bar, sizeof(unsigned))) ||
@@ -1731,6 +1763,10 @@ int cpfft_init(int N, const int* matList, const double* kocks_deg, const cpfft_c
       cudaMallocHost((void**)&c->h_stats, 8 * sizeof(unsigned long long)) != cudaSuccess) {
     cpfft_set_error("cudaMallocHost failed");
     return fail(CPFFT_ERR_NO_MEMORY);
+  }
+  for (int k = 0; k < ncrystals; k++) {
+    if (tab_n1[k] >= 0) cr[k].tab_n1 = c->ptabs + tab_n1[k];
+    if (tab_c8[k] >= 0) cr[k].tab_c8 = c->ptabs + tab_c8[k];
   }
   std::vector<double2> tw(N);
   for (int k = 0; k < N; k++) {
@@ -1768,6 +1804,8 @@ int cpfft_init(int N, const int* matList, const double* kocks_deg, const cpfft_c
       (e = cudaMemcpy(c->crys, crys.data(), N3 * sizeof(int), cudaMemcpyHostToDevice)) ||
       (e = cudaMemcpy(c->oris, oris.data(), oris.size() * sizeof(OriRec), cudaMemcpyHostToDevice)) ||
       (e = cudaMemcpy(c->cryss, cr.data(), ncrystals * sizeof(CrysRec), cudaMemcpyHostToDevice)) ||
+      (tabs.size() && (e = cudaMemcpy(c->ptabs, tabs.data(), tabs.size() * sizeof(PowTab),
+                                      cudaMemcpyHostToDevice))) ||
       (e = green_setup<double>(N))) {
     cpfft_set_error("cpfft_init: %s", cudaGetErrorString(e));
     return fail(CPFFT_ERR_CUDA);

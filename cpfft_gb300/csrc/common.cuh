@@ -37,6 +37,17 @@ struct OriRec {
   double g[9];     // lattice -> sample rotation applied to b and n, row-major
 };
 
+// Table of x^y for a fixed exponent 0 < y <= 8 (tpow, stress.cu; filled by pow_table,
+// api.cu): x = 2^k m, c the midpoint of m's interval of [1, 2).
+struct PowTab {
+  static constexpr int NM = 256, NE = 1024, EMID = 512;
+  double y;
+  double c[6];     // binomial coefficients y, y (y - 1) / 2, .. of (1 + u)^y - 1
+  double rc[NM];   // 1 / c, rounded
+  double P[NM];    // rc^-y
+  double E[NE];    // 2^(y (k - EMID))
+};
+
 // Scalars of one crystal definition that the Voce path reads.
 struct CrysRec {
   double rate_n, tau_y, tau_v, inv_tau_v, theta_0, voce_m, gamma_bar, iD_v;
@@ -52,6 +63,9 @@ struct CrysRec {
   int miter, alter_mode, exact_j22;
   int n_int;       // rate_n - 1 when rate_n is integer-valued in [2, 64], else -1
   int m_is_one;    // voce_m == 1
+  // tables of |x|^(rate_n - 1) (n_int < 0) and of gd^c8 (MRR, ORNL), null where the exponent
+  // has none
+  const PowTab *tab_n1, *tab_c8;
 };
 
 // One bilinear Mises material (mm01, src/mm01.f; properties of setup_mm01_rknstr,

@@ -5,10 +5,15 @@
 // strain increment, the mm10 Voce/FCC crystal update (src/mm10_a.f, src/mm10_b.f), the
 // Cauchy -> first Piola-Kirchhoff pull-back and the exact dP/dF of cep2A
 // (src/cep2A.f:86-284).  The arithmetic is reorganised for a GPU whose FP64 pipe is
-// the bound: integer powers by binary powering when the rate exponent is integral,
-// reciprocals hoisted out of the 12-slip loops, and cep2A's 81-term loops contracted
-// through 3x3 intermediates (about 1.6 kflop instead of ~20 kflop).  Every local loop
-// is bounded by miter and the line-search cap, so no thread can spin.
+// the bound: an FP64 warp instruction holds its SM quarter for 64 clocks whatever its active
+// lanes, a division costs six of them, a square root ten and CUDA's pow about 95.  Powers are
+// binary powering (integral rate exponents) or a table per exponent (tpow), divisions and
+// square roots are hoisted or avoided, each residual keeps its slips for the Jacobian, the
+// tangent and the rotation, contractions with the trace-free Schmid tensors take five
+// products, and cep2A's 81-term loops are contracted through 3x3 intermediates (about 1.6
+// kflop instead of ~20 kflop).  One implicit pass with the reference's start on a GB300: 64^3
+// FCC Voce 22.5 to 15.7 ms, 32^3 BCC-48 (exponent 5.48) 12.3 to 4.4 ms.  Every local loop is
+// bounded by miter and the line-search cap, so no thread can spin.
 #include <algorithm>
 
 #include "common.cuh"
@@ -41,18 +46,40 @@ constexpr double TEMP = 297.0;
 
 __device__ __forceinline__ double sgn1(double x) { return x < 0.0 ? -1.0 : 1.0; }
 
-// |x|^e for a non-negative integer e by binary powering
+// x^e for an integer e >= 1 by binary powering
 __device__ __forceinline__ double ipow(double x, int e) {
-  double r = 1.0, b = x;
-  while (e) {
-    if (e & 1) r *= b;
-    b *= b;
-    e >>= 1;
+  while (!(e & 1)) { x *= x; e >>= 1; }
+  double r = x;
+  while (e >>= 1) {
+    x *= x;
+    if (e & 1) r *= x;
   }
   return r;
 }
-__device__ __forceinline__ double powabs(double x, int n_int, double e) {
-  return n_int >= 0 ? ipow(fabs(x), n_int) : pow(fabs(x), e);
+// x^y, x >= 0, with the exponent's table: x = 2^k m, the interval's 1/c from m's leading bits,
+// u = m / c - 1 (one rounding), c^y 2^(y k) ((1 + u)^y by its binomial series, |u| <= 2^-9).
+// Nine FP64 instructions where CUDA's pow takes about 95; error at most 2.5 ulp over the table's
+// range (0 < y <= 8, 2^-512 <= x < 2^512; pow elsewhere).
+__device__ __forceinline__ double tpow(const PowTab* __restrict__ t, double x) {
+  const int hi = __double2hiint(x);
+  const unsigned k = (unsigned)((hi >> 20) - 1023 + PowTab::EMID);
+  if (k >= PowTab::NE) return x == 0.0 ? 0.0 : pow(x, t->y);
+  const int i = (hi >> 12) & (PowTab::NM - 1);
+  const double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(x));
+  const double u = fma(m, __ldg(t->rc + i), -1.0);
+  const double w = __ldg(t->P + i) * __ldg(t->E + k);
+  double q = __ldg(t->c + 5);
+#pragma unroll
+  for (int j = 4; j >= 0; j--) q = fma(q, u, __ldg(t->c + j));
+  return fma(w, q * u, w);
+}
+// |x|^(n-1) and x^n (x > 0) for the crystal's rate exponent n
+__device__ __forceinline__ double pow_n1(const CrysRec& c, double x) {
+  x = fabs(x);
+  return c.n_int >= 0 ? ipow(x, c.n_int) : c.tab_n1 ? tpow(c.tab_n1, x) : pow(x, c.rate_n - 1.0);
+}
+__device__ __forceinline__ double pow_n(const CrysRec& c, double x) {
+  return c.n_int >= 0 ? ipow(x, c.n_int + 1) : c.tab_n1 ? x * tpow(c.tab_n1, x) : pow(x, c.rate_n);
 }
 
 // ---- 3x3 helpers (row-major [9]; FP64, or FP32 for the fast form's tangent) ------------
@@ -196,9 +223,11 @@ __device__ __forceinline__ void symsw(const double* s, const double* w, double* 
   sw[5] = 0.5 * (w[1] * (s[0] - s[2]) + w[0] * s[3] - w[2] * s[4]);
 }
 
-// LU with partial pivoting, in place, n <= 7, one right-hand side
+// LU with partial pivoting, in place, n <= 18, one right-hand side.  The pivots'
+// reciprocals are formed once (a division costs about six FP64 instructions).
 template <int n>
 __device__ bool lu_solve1(double* a, double* b) {
+  double inv[n];
   for (int k = 0; k < n; k++) {
     int p = k;
     double best = fabs(a[k * n + k]);
@@ -208,13 +237,12 @@ __device__ bool lu_solve1(double* a, double* b) {
     }
     if (best == 0.0) return false;
     if (p != k) {
-      for (int j = 0; j < n; j++) { double t = a[k * n + j]; a[k * n + j] = a[p * n + j]; a[p * n + j] = t; }
+      for (int j = k; j < n; j++) { double t = a[k * n + j]; a[k * n + j] = a[p * n + j]; a[p * n + j] = t; }
       double t = b[k]; b[k] = b[p]; b[p] = t;
     }
-    double inv = 1.0 / a[k * n + k];
+    inv[k] = 1.0 / a[k * n + k];
     for (int i = k + 1; i < n; i++) {
-      double l = a[i * n + k] * inv;
-      a[i * n + k] = l;
+      double l = a[i * n + k] * inv[k];
       for (int j = k + 1; j < n; j++) a[i * n + j] -= l * a[k * n + j];
       b[i] -= l * b[k];
     }
@@ -222,7 +250,7 @@ __device__ bool lu_solve1(double* a, double* b) {
   for (int i = n - 1; i >= 0; i--) {
     double s = b[i];
     for (int k = i + 1; k < n; k++) s -= a[i * n + k] * b[k];
-    b[i] = s / a[i * n + i];
+    b[i] = s * inv[i];
   }
   return true;
 }
@@ -240,6 +268,8 @@ struct Crystal {
   double ms[NS][6];
   double qc[NS][3];
   double Cms[NS][6];  // C ms_i, constant while ms is (the reference forms it per call)
+  // the last residual's resolved shears, slip increments, |rs|^(n-1) and dg / tt^n
+  double rs[NS], si[NS], pw[NS], dgn;
   // MTS: shear modulus and thresholds of this (sub)step, the n-state values of the history's
   // u words (nu1, nu2 < 0: first step), and the temperature of the (sub)step
   double mu, tau_y, tau_v, ntau_y, nmu, nu1, nu2, temp;
@@ -266,6 +296,11 @@ __device__ void setup_np1(Crystal& s, const OriRec* rec, const double* D, double
   rt2rve(tr, RE);
   mm3(R, tr, work);
   rt2rvw(work, RWC);
+  double c0[6], c1[6];
+  for (int a = 0; a < 6; a++) {
+    c0[a] = Cv(s.C, a, 0) - Cv(s.C, a, 2);
+    c1[a] = Cv(s.C, a, 1) - Cv(s.C, a, 2);
+  }
   for (int i = 0; i < NS; i++) {
     double m0[6], q0[3];
     for (int a = 0; a < 6; a++) m0[a] = __ldg(rec->ms + 6 * i + a);
@@ -277,29 +312,30 @@ __device__ void setup_np1(Crystal& s, const OriRec* rec, const double* D, double
     }
     for (int a = 0; a < 3; a++)
       s.qc[i][a] = RWC[3 * a] * q0[0] + RWC[3 * a + 1] * q0[1] + RWC[3 * a + 2] * q0[2];
-    for (int a = 0; a < 6; a++) {
-      double v = 0.0;
-      for (int j = 0; j < 6; j++) v += Cv(s.C, a, j) * s.ms[i][j];
-      s.Cms[i][a] = v;
-    }
+    // the first three components of ms sum to zero (b . n = 0, kept by the rotation), so every
+    // contraction with ms takes five products: sum_j v_j ms_j = (v_0 - v_2) ms_0 + (v_1 - v_2)
+    // ms_1 + v_3 ms_3 + v_4 ms_4 + v_5 ms_5
+    for (int a = 0; a < 6; a++)
+      s.Cms[i][a] = c0[a] * s.ms[i][0] + c1[a] * s.ms[i][1] + Cv(s.C, a, 3) * s.ms[i][3] +
+                    Cv(s.C, a, 4) * s.ms[i][4] + Cv(s.C, a, 5) * s.ms[i][5];
   }
 }
 
 // resolved shear and slip increment of every system (mm10_rs, mm10_slipinc):
 //   si = dg/tt |rs/tt|^(n-1) rs = dg |rs|^(n-1) rs / tt^n,
-// keeping pw = |rs|^(n-1), which the Jacobian reuses (d si / d rs, d si / d tt)
-__device__ __forceinline__ void slips(const Crystal& s, const double* st, double tt, double* rs,
-                                      double* si, double* pw) {
+// keeping pw = |rs|^(n-1) and dgn = dg / tt^n, which the Jacobian reuses (d si / d rs,
+// d si / d tt)
+__device__ __forceinline__ void slips(Crystal& s, const double* st, double tt) {
   const CrysRec& c = *s.cr;
-  double itt = 1.0 / tt;
-  double dgn = s.dg * (c.n_int >= 0 ? ipow(itt, c.n_int + 1) : pow(itt, c.rate_n));
+  s.dgn = s.dg * pow_n(c, 1.0 / tt);
+  const double d0 = st[0] - st[2], d1 = st[1] - st[2];
   for (int i = 0; i < NS; i++) {
-    double r = st[0] * s.ms[i][0] + st[1] * s.ms[i][1] + st[2] * s.ms[i][2] +
-               st[3] * s.ms[i][3] + st[4] * s.ms[i][4] + st[5] * s.ms[i][5];
-    rs[i] = r;
-    double p = powabs(r, c.n_int, c.rate_n - 1.0);
-    pw[i] = p;
-    si[i] = dgn * p * r;
+    const double r = d0 * s.ms[i][0] + d1 * s.ms[i][1] + st[3] * s.ms[i][3] + st[4] * s.ms[i][4] +
+                     st[5] * s.ms[i][5];
+    const double p = pow_n1(c, r);
+    s.rs[i] = r;
+    s.pw[i] = p;
+    s.si[i] = s.dgn * p * r;
   }
 }
 
@@ -344,17 +380,19 @@ __device__ __forceinline__ double hpow(const CrysRec& c, double h) {
   return c.m_is_one ? fabs(h) : pow(fabs(h), c.voce_m);
 }
 
-// R1 (mm10_formR1, src/mm10_b.f:1061-1101) from precomputed rs / slip increments
-__device__ void formR1(const Crystal& s, const double* st, const double* rs, const double* si,
-                       double* R1) {
+// R1 (mm10_formR1, src/mm10_b.f:1061-1101) from the last slips
+__device__ void formR1(const Crystal& s, const double* st, double* R1) {
   const CrysRec& c = *s.cr;
   double dbar[6] = {0, 0, 0, 0, 0, 0}, w[3] = {0, 0, 0};
   double tid = s.tinc * c.iD_v;
   for (int i = 0; i < NS; i++) {
-    double f = rs[i] * tid + si[i];
-    for (int a = 0; a < 6; a++) dbar[a] += f * s.ms[i][a];
+    const double f = s.rs[i] * tid + s.si[i];
+    dbar[0] += f * s.ms[i][0];
+    dbar[1] += f * s.ms[i][1];
+    for (int a = 3; a < 6; a++) dbar[a] += f * s.ms[i][a];
     for (int a = 0; a < 3; a++) w[a] += f * s.qc[i][a];
   }
+  dbar[2] = -(dbar[0] + dbar[1]);
   double sw[6], wv[6];
   symsw(st, w, sw);
   for (int a = 0; a < 6; a++) wv[a] = s.D[a] - dbar[a];
@@ -365,56 +403,72 @@ __device__ void formR1(const Crystal& s, const double* st, const double* rs, con
   }
 }
 
-// full residual (mm10_formR + mm10_formR2 / mm10_h_voche); returns tau_tilde rate
-__device__ double formR(const Crystal& s, const double* x, double* R, double* rs, double* si,
-                        double* pw) {
+// R2 (mm10_formR2 / mm10_h_voche) from the last slips; returns the tau_tilde rate
+__device__ double formR2(const Crystal& s, double tt, double* R2) {
   const CrysRec& c = *s.cr;
-  slips(s, x, x[6], rs, si, pw);
-  formR1(s, x, rs, si, R);
-  double h = 0.0;
+  double g = 0.0, h;
+  for (int i = 0; i < NS; i++) g += fabs(s.si[i]);
   if constexpr (MTS) {  // mm10_h_mts (src/mm10_b.f:2080-2108)
-    const double hp = pow(mts_base(s, mts_cta(s, x[6])), c.voce_m);
-    for (int i = 0; i < NS; i++) h += hp * fabs(si[i]);
+    h = pow(mts_base(s, mts_cta(s, tt)), c.voce_m) * g;
     h = c.tau_a * (1.0 - s.mu / s.nmu) + (s.mu / c.mu_0) * (s.tau_y - s.ntau_y) +
         (s.mu / s.nmu) * s.ntt + c.theta_0 * (s.mu / c.mu_0) * h;
   } else {
-    double ht = hterm(c, x[6]);
-    double hp = hpow(c, ht) * sgn1(ht);
-    for (int i = 0; i < NS; i++) h += hp * fabs(si[i]);
-    h = s.ntt + c.theta_0 * h;
+    const double ht = hterm(c, tt);
+    h = s.ntt + c.theta_0 * (hpow(c, ht) * sgn1(ht) * g);
   }
-  R[6] = x[6] - h;
+  *R2 = tt - h;
   return (h - s.ntt) / s.tinc;
 }
 
-// J11 (mm10_formJ11, src/mm10_b.f:177-257); J is 6x6 row-major inside a 7x7 when ld=7
+// full residual (mm10_formR); returns the tau_tilde rate
+__device__ double formR(Crystal& s, const double* x, double* R) {
+  slips(s, x, x[6]);
+  formR1(s, x, R);
+  return formR2(s, x[6], R + 6);
+}
+
+// J11 (mm10_formJ11, src/mm10_b.f:177-257) at the last slips; J is 6x6 row-major inside a
+// 7x7 when ld=7
 template <int ld, bool WITH12>
-__device__ void formJ11(const Crystal& s, const double* st, double tt, const double* rs,
-                        const double* si, const double* pw, double* J, double* J12,
-                        double itt) {
+__device__ void formJ11(const Crystal& s, const double* st, double* J, double* J12, double itt) {
   const CrysRec& c = *s.cr;
   for (int a = 0; a < 6; a++)
     for (int b = 0; b < 6; b++) J[ld * a + b] = 0.0;
   // d si / d rs = dg n |rs|^(n-1) / tt^n (mm10_dgdt_voche)
-  double fac = s.dg * c.rate_n / (c.n_int >= 0 ? ipow(tt, c.n_int + 1) : pow(tt, c.rate_n));
-  double tid = s.tinc * c.iD_v;
+  const double fac = s.dgn * c.rate_n, tid = s.tinc * c.iD_v;
+  const double nt = -c.rate_n * itt;  // d si / d tt = -n si / tt (mm10_dgdh_voche)
   double w[3] = {0, 0, 0};
+  // 2 symsw(st, q) with the stress differences formed once
+  const double t3 = 2.0 * st[3], t4 = 2.0 * st[4], t5 = 2.0 * st[5];
+  const double d01 = st[0] - st[1], d12 = st[1] - st[2], d02 = st[0] - st[2];
   for (int i = 0; i < NS; i++) {
-    double dgdt = fac * pw[i] + tid;
-    double sq[6], wv[6];
-    symsw(st, s.qc[i], sq);
-    for (int a = 0; a < 6; a++) wv[a] = s.Cms[i][a] + 2.0 * sq[a];
+    const double dgdt = fac * s.pw[i] + tid;
+    const double q0 = s.qc[i][0], q1 = s.qc[i][1], q2 = s.qc[i][2];
+    double wv[6];
+    wv[0] = s.Cms[i][0] + t3 * q2 - t5 * q1;
+    wv[1] = s.Cms[i][1] + t3 * q2 - t4 * q0;
+    wv[2] = s.Cms[i][2] + t5 * q1 + t4 * q0;
+    wv[3] = s.Cms[i][3] + q2 * d01 + q0 * st[5] - q1 * st[4];
+    wv[4] = s.Cms[i][4] + q0 * d12 + q1 * st[3] + q2 * st[5];
+    wv[5] = s.Cms[i][5] + q1 * d02 + q0 * st[3] - q2 * st[4];
+    // column 2 is minus the sum of columns 0 and 1 (ms is trace free): formed after the loop
+#pragma unroll
     for (int b = 0; b < 6; b++) {
-      double t = dgdt * s.ms[i][b];
+      if (b == 2) continue;
+      const double t = dgdt * s.ms[i][b];
+#pragma unroll
       for (int a = 0; a < 6; a++) J[ld * a + b] += wv[a] * t;
     }
     if (WITH12) {  // the same (C ms + 2 symTW) vector drives J12 (mm10_formJ12)
-      double dgdtt = -c.rate_n * itt * si[i];  // mm10_dgdh_voche
+      const double dgdtt = nt * s.si[i];
       for (int a = 0; a < 6; a++) J12[a] += wv[a] * dgdtt;
     }
-    double f = rs[i] * tid + si[i];
-    for (int a = 0; a < 3; a++) w[a] += f * s.qc[i][a];
+    const double f = s.rs[i] * tid + s.si[i];
+    w[0] += f * q0;
+    w[1] += f * q1;
+    w[2] += f * q2;
   }
+  for (int a = 0; a < 6; a++) J[ld * a + 2] = -(J[ld * a] + J[ld * a + 1]);
   // mm10_iw (src/mm10_b.f:1590-1634) and the identity
   J[ld * 0 + 3] += 2.0 * w[2];  J[ld * 0 + 5] -= 2.0 * w[1];
   J[ld * 1 + 3] += 2.0 * w[2];  J[ld * 1 + 4] -= 2.0 * w[0];
@@ -425,59 +479,48 @@ __device__ void formJ11(const Crystal& s, const double* st, double tt, const dou
   for (int a = 0; a < 6; a++) J[ld * a + a] += 1.0;
 }
 
-// full 7x7 Jacobian (mm10_formJ, src/mm10_b.f:901-954)
-__device__ void formJ(const Crystal& s, const double* x, const double* rs, const double* si,
-                      const double* pw, double* J) {
+// full 7x7 Jacobian (mm10_formJ, src/mm10_b.f:901-954) at the last slips
+__device__ void formJ(const Crystal& s, const double* x, double* J) {
   const CrysRec& c = *s.cr;
-  double tt = x[6];
-  double itt = 1.0 / tt;
+  const double tt = x[6], itt = 1.0 / tt;
   double J12[6] = {0, 0, 0, 0, 0, 0}, et[6] = {0, 0, 0, 0, 0, 0};
-  formJ11<7, true>(s, x, tt, rs, si, pw, J, J12, itt);
+  formJ11<7, true>(s, x, J, J12, itt);
+  // sum of |rs|^(n-1) sign(rs) ms (mm10_estress_*), of |si| and of |si| sign(1, si)
+  double g = 0.0, gs = 0.0;
+  for (int i = 0; i < NS; i++) {
+    const double r2 = copysign(s.pw[i], s.rs[i]);
+    et[0] += r2 * s.ms[i][0];
+    et[1] += r2 * s.ms[i][1];
+    for (int a = 3; a < 6; a++) et[a] += r2 * s.ms[i][a];
+    g += fabs(s.si[i]);
+    gs += s.si[i];
+  }
+  et[2] = -(et[0] + et[1]);
+  if (c.n_int < 0 && c.rate_n < 2.0) {  // |rs|^(n-2) rs of the reference: NaN at rs = 0
+    for (int i = 0; i < NS; i++)
+      if (s.rs[i] == 0.0) et[0] = __longlong_as_double(0x7ff8000000000000ULL);
+  }
+  double fac;
   if constexpr (MTS) {
     // mm10_estress_mts / mm10_ehard_mts (src/mm10_b.f:2110-2187)
     const double cta = mts_cta(s, tt);
     const double b = mts_base(s, cta);
     const double bm = pow(b, c.voce_m);
     const double ur = s.mu / c.mu_0;
-    double sum = 0.0;
-    for (int i = 0; i < NS; i++) {
-      double r2 = c.n_int >= 0 ? (rs[i] < 0.0 ? -pw[i] : (rs[i] > 0.0 ? pw[i] : 0.0))
-                               : pow(fabs(rs[i]), c.rate_n - 2.0) * rs[i];
-      for (int a = 0; a < 6; a++) et[a] += bm * r2 * s.ms[i][a];
-      sum += (c.voce_m * (1.0 / s.tau_v + 0.0 / (cta * cta)) * pow(b, -1.0) +
-              ur * c.rate_n / tt) * bm * fabs(si[i]);
-    }
-    const double fac = c.theta_0 * ur * c.rate_n * s.dg /
-                       (c.n_int >= 0 ? ipow(tt, c.n_int + 1) : pow(tt, c.rate_n));
-    for (int a = 0; a < 6; a++) {
-      J[7 * a + 6] = J12[a];
-      J[7 * 6 + a] = -(fac * et[a]);
-    }
-    J[48] = 1.0 + c.theta_0 * sum;
-    return;
+    fac = c.theta_0 * ur * c.rate_n * s.dgn * bm;
+    J[48] = 1.0 + c.theta_0 * ((c.voce_m * (1.0 / s.tau_v + 0.0 / (cta * cta)) / b + ur * c.rate_n * itt) * bm * g);
+  } else {
+    const double ht = hterm(c, tt), hp = hpow(c, ht), sh = sgn1(ht);
+    // mm10_ehard_voche; exact_j22 = 0 keeps the reference's extra sign(1, si)
+    const double ta = c.voce_m * (-c.inv_tau_v) / fabs(ht) * g;
+    const double tb = c.rate_n * itt * sh * (c.exact_j22 ? g : gs);
+    fac = c.theta_0 * s.dgn * c.rate_n * hp * sh;
+    J[48] = 1.0 - c.theta_0 * ((ta - tb) * hp);
   }
-  double ht = hterm(c, tt);
-  double hp = hpow(c, ht);
-  double sh = sgn1(ht);
-  double etau = 0.0;
-  for (int i = 0; i < NS; i++) {
-    // mm10_estress_voche: |rs|^(n-2) rs = |rs|^(n-1) sign(rs)
-    double r2 = c.n_int >= 0 ? (rs[i] < 0.0 ? -pw[i] : (rs[i] > 0.0 ? pw[i] : 0.0))
-                             : pow(fabs(rs[i]), c.rate_n - 2.0) * rs[i];
-    double f = hp * sh * r2;
-    for (int a = 0; a < 6; a++) et[a] += f * s.ms[i][a];
-    double asi = fabs(si[i]);                          // mm10_ehard_voche
-    double ta = c.voce_m * (-c.inv_tau_v) * asi / fabs(ht);
-    double tb = asi * c.rate_n * itt * sh;
-    if (!c.exact_j22) tb *= sgn1(si[i]);
-    etau += (ta - tb) * hp;
-  }
-  double fac = c.theta_0 * s.dg * c.rate_n / (c.n_int >= 0 ? ipow(tt, c.n_int + 1) : pow(tt, c.rate_n));
   for (int a = 0; a < 6; a++) {
     J[7 * a + 6] = J12[a];
     J[7 * 6 + a] = -(fac * et[a]);
   }
-  J[48] = 1.0 - c.theta_0 * etau;
 }
 
 // mm10_tangent's JA and JB for MTS (src/mm10_a.f:658-815 with mm10_ed_mts and
@@ -485,11 +528,10 @@ __device__ void formJ(const Crystal& s, const double* x, const double* rs, const
 // JR -= JA + JB, JA = sum_i (C ms_i + 2 symtq) (x) dgamma_i/dD, JB = J12 (x) ed / J22.
 // The reference passes the whole symtqmat where a column is meant, so every system's JA
 // term takes system 1's column (mm10_a_mult_type_4 reads its first six words).
+// The slips are the last residual's, which is the converged state's.
 __device__ void mts_tangent_rhs(const Crystal& s, const double* st, double tt, const double* J,
                                 double* JR) {
   const CrysRec& c = *s.cr;
-  double rs[NS], si[NS], pw[NS];
-  slips(s, st, tt, rs, si, pw);
   const double dm[6] = {s.D[0], s.D[1], s.D[2], 0.5 * s.D[3], 0.5 * s.D[4], 0.5 * s.D[5]};
   const double alpha = 2.0 / (3.0 * s.dg * s.dg);
   double sq1[6];
@@ -498,7 +540,7 @@ __device__ void mts_tangent_rhs(const Crystal& s, const double* st, double tt, c
   for (int i = 0; i < NS; i++) {
     double wv[6];
     for (int a = 0; a < 6; a++) wv[a] = s.Cms[i][a] + 2.0 * sq1[a];
-    const double g = alpha * si[i];
+    const double g = alpha * s.si[i];
     for (int a = 0; a < 6; a++)
       for (int b = 0; b < 6; b++) JR[6 * a + b] -= wv[a] * (g * dm[b]);
   }
@@ -519,7 +561,7 @@ __device__ void mts_tangent_rhs(const Crystal& s, const double* st, double tt, c
   const double bm1 = pow(base, c.voce_m - 1.0), bm = pow(base, c.voce_m);
   double ky = 0.0, kv = 0.0, kd = 0.0;
   for (int i = 0; i < NS; i++) {
-    const double asi = fabs(si[i]);
+    const double asi = fabs(s.si[i]);
     ky += c.voce_m * (1.0 / s.tau_v + 0.0 / (sc * sc)) * bm1 * asi;
     kv += c.voce_m / (s.tau_v * s.tau_v) * sc * bm1 * asi;
     kd += 2.0 / (3.0 * s.dg * s.dg) * bm * asi;
@@ -539,9 +581,18 @@ __device__ __forceinline__ bool anynan(const double* x, int n) {
   return r;
 }
 
-__device__ bool newton_update(Crystal& cu, double* x, double inR_alt, double* Jlast, bool& haveJ,
-                              int& iters, double& ttrate, bool fixed_scale = false,
-                              int cap = 1 << 30);
+__device__ bool newton_update(Crystal& cu, double* x, double inR2_alt, double* Jlast, bool& haveJ,
+                              int& iters, double& ttrate, const double* R1 = nullptr,
+                              bool fixed_scale = false, int cap = 1 << 30);
+
+// ||v||^2 (the stop tests compare squares: a square root and a division are 15 FP64
+// instructions)
+template <int n>
+__device__ __forceinline__ double norm2(const double* v) {
+  double d = 0;
+  for (int a = 0; a < n; a++) d += v[a] * v[a];
+  return d;
+}
 
 // tau_tilde extrapolated along the previous step's rate (mm10_solve, src/mm10_a.f:2900-2935):
 // tau_n + max(cos(dev D, dev D_n), 0) * tau_rate_n * dt
@@ -563,62 +614,47 @@ __device__ double tau_extrapolated(const Crystal& cu, double tt, double dtinc) {
 
 // mm10_solve (src/mm10_a.f:2860-3295): predict on R1 with tau_tilde extrapolated, then
 // the coupled Newton; Armijo line search c = 1e-4, halving, at most 11 trials.
+// The Newton direction solves J dx = -R, so the Armijo slope dx . J^T R is -||R||^2.
 __device__ bool solve(Crystal& cu, double dtinc, double* stress, double& tt, double* Jlast,
                       bool& haveJ, int& iters, int& piters, double& ttrate) {
   const CrysRec& c = *cu.cr;
   const double cls = 1.0e-4;
-  double x[7], rs[NS], si[NS], pw[NS];
+  double x[7], R1[6], inR2;
   for (int i = 0; i < 6; i++) x[i] = stress[i];
-  x[6] = tt;
-  double inR1;
+  x[6] = tau_extrapolated(cu, tt, dtinc);
   {  // ---- predict
-    double x2 = tau_extrapolated(cu, x[6], dtinc);
-    double x1[6], R1[6];
-    for (int i = 0; i < 6; i++) x1[i] = x[i];
-    slips(cu, x1, x2, rs, si, pw);
-    formR1(cu, x1, rs, si, R1);
-    double dot = 0;
-    for (int a = 0; a < 6; a++) dot += R1[a] * R1[a];
-    double nR1 = sqrt(dot);
-    inR1 = nR1;
+    slips(cu, x, x[6]);
+    formR1(cu, x, R1);
+    double dot = norm2<6>(R1);
+    inR2 = dot;
+    const double stop = fmax(c.atol1 * c.atol1, c.rtol1 * c.rtol1 * inR2);
     int it = 0;
-    while (nR1 > c.atol1 && nR1 / inR1 > c.rtol1) {
-      double J[36], mJ[36], dx[6];
-      formJ11<6, false>(cu, x1, x2, rs, si, pw, J, nullptr, 0.0);
-      for (int a = 0; a < 36; a++) mJ[a] = -J[a];
-      for (int a = 0; a < 6; a++) dx[a] = R1[a];
-      lu_solve1<6>(mJ, dx);
-      double ls1 = 0.5 * dot, ls2 = 0.0;
-      for (int a = 0; a < 6; a++) {
-        double wv = 0.0;
-        for (int b = 0; b < 6; b++) wv += J[6 * b + a] * R1[b];
-        ls2 += dx[a] * wv;
-      }
-      ls2 *= cls;
+    while (dot > stop) {
+      double J[36], dx[6];
+      formJ11<6, false>(cu, x, J, nullptr, 0.0);
+      for (int a = 0; a < 6; a++) dx[a] = -R1[a];
+      lu_solve1<6>(J, dx);
+      const double ls1 = 0.5 * dot, ls2 = -cls * dot;
       double alpha = 1.0;
       for (int ls = 0;; ls++) {
         double xn[6];
-        for (int a = 0; a < 6; a++) xn[a] = x1[a] + alpha * dx[a];
-        slips(cu, xn, x2, rs, si, pw);
-        formR1(cu, xn, rs, si, R1);
-        dot = 0;
-        for (int a = 0; a < 6; a++) dot += R1[a] * R1[a];
-        nR1 = sqrt(dot);
+        for (int a = 0; a < 6; a++) xn[a] = x[a] + alpha * dx[a];
+        slips(cu, xn, x[6]);
+        formR1(cu, xn, R1);
+        dot = norm2<6>(R1);
         if (0.5 * dot <= ls1 + ls2 * alpha || ls > 10) {
-          for (int a = 0; a < 6; a++) x1[a] = xn[a];
+          for (int a = 0; a < 6; a++) x[a] = xn[a];
           break;
         }
         alpha *= 0.5;
       }
       it++;
-      if (it > c.miter || anynan(x1, 6)) { piters += it; return false; }
+      if (it > c.miter || anynan(x, 6)) { piters += it; return false; }
     }
     piters += it;
-    for (int i = 0; i < 6; i++) x[i] = x1[i];
-    x[6] = x2;
   }
-  // ---- update
-  if (!newton_update(cu, x, inR1, Jlast, haveJ, iters, ttrate)) return false;
+  // ---- update, from the predictor's state (its slips and R1 are current)
+  if (!newton_update(cu, x, inR2, Jlast, haveJ, iters, ttrate, R1)) return false;
   for (int i = 0; i < 6; i++) stress[i] = x[i];
   tt = x[6];
   return true;
@@ -650,16 +686,14 @@ __device__ void pull_inside(const Crystal& cu, const double* nsig, double* x, do
 __device__ bool solve_from(Crystal& cu, double dtinc, const double* x0, double* stress,
                            double& tt, double* Jlast, bool& haveJ, int& iters, double& ttrate,
                            int cap) {
-  double x[7], R[7], rs[NS], si[NS], pw[NS];
+  double x[7], R[7];
   for (int i = 0; i < 6; i++) x[i] = stress[i];
   x[6] = tau_extrapolated(cu, tt, dtinc);
-  formR(cu, x, R, rs, si, pw);
-  double dot = 0;
-  for (int a = 0; a < 7; a++) dot += R[a] * R[a];
-  const double scale = sqrt(dot);
+  formR(cu, x, R);
+  const double scale2 = norm2<7>(R);
   for (int i = 0; i < 7; i++) x[i] = x0[i];
   if (!(x[6] > 0.0) || anynan(x, 7)) return false;
-  if (!newton_update(cu, x, scale, Jlast, haveJ, iters, ttrate, true, cap)) return false;
+  if (!newton_update(cu, x, scale2, Jlast, haveJ, iters, ttrate, nullptr, true, cap)) return false;
   for (int i = 0; i < 6; i++) stress[i] = x[i];
   tt = x[6];
   return true;
@@ -667,44 +701,41 @@ __device__ bool solve_from(Crystal& cu, double dtinc, const double* x0, double* 
 
 // The coupled 7x7 Newton of mm10_solve (src/mm10_a.f:3105-3295) from x = (sigma, tau):
 // Armijo line search, converged when ||R|| <= atol or ||R|| / ||R_0|| <= rtol after at
-// least one iteration; inR_alt replaces ||R_0|| when the start is an exact root.
-// fixed_scale: inR_alt is the relative test's scale (a start other than the predictor's);
-// cap: an iteration limit below miter (that start is then abandoned)
-__device__ bool newton_update(Crystal& cu, double* x, double inR_alt, double* Jlast, bool& haveJ,
-                              int& iters, double& ttrate, bool fixed_scale, int cap) {
+// least one iteration; inR2_alt replaces ||R_0||^2 when the start is an exact root.
+// R1 (6): the stress residual at x when the slips are already x's; fixed_scale: inR2_alt is
+// the relative test's scale (a start other than the predictor's); cap: an iteration limit
+// below miter (that start is then abandoned)
+__device__ bool newton_update(Crystal& cu, double* x, double inR2_alt, double* Jlast, bool& haveJ,
+                              int& iters, double& ttrate, const double* R1, bool fixed_scale,
+                              int cap) {
   const CrysRec& c = *cu.cr;
   const double cls = 1.0e-4;
-  double rs[NS], si[NS], pw[NS];
   int it = 0;
   double R[7];
-  ttrate = formR(cu, x, R, rs, si, pw);
-  double dot = 0;
-  for (int a = 0; a < 7; a++) dot += R[a] * R[a];
-  double nR = sqrt(dot), inR = nR;
-  if (inR == 0.0 || fixed_scale) inR = inR_alt;
+  if (R1) {
+    for (int a = 0; a < 6; a++) R[a] = R1[a];
+    ttrate = formR2(cu, x[6], R + 6);
+  } else {
+    ttrate = formR(cu, x, R);
+  }
+  double dot = norm2<7>(R), inR2 = dot;
+  if (inR2 == 0.0 || fixed_scale) inR2 = inR2_alt;
+  const double stop = fmax(c.atol * c.atol, c.rtol * c.rtol * inR2);
   const int mit = min(c.miter, cap);
-  while ((nR > c.atol && nR / inR > c.rtol) || it < 1) {
-    formJ(cu, x, rs, si, pw, Jlast);
+  while (dot > stop || it < 1) {
+    formJ(cu, x, Jlast);
     haveJ = true;
     double mJ[49], dx[7];
-    for (int a = 0; a < 49; a++) mJ[a] = -Jlast[a];
-    for (int a = 0; a < 7; a++) dx[a] = R[a];
+    for (int a = 0; a < 49; a++) mJ[a] = Jlast[a];
+    for (int a = 0; a < 7; a++) dx[a] = -R[a];
     lu_solve1<7>(mJ, dx);
-    double ls1 = 0.5 * dot, ls2 = 0.0;
-    for (int a = 0; a < 7; a++) {
-      double wv = 0.0;
-      for (int b = 0; b < 7; b++) wv += Jlast[7 * b + a] * R[b];
-      ls2 += dx[a] * wv;
-    }
-    ls2 *= cls;
+    const double ls1 = 0.5 * dot, ls2 = -cls * dot;
     double alpha = 1.0;
     for (int ls = 0;; ls++) {
       double xn[7];
       for (int a = 0; a < 7; a++) xn[a] = x[a] + alpha * dx[a];
-      ttrate = formR(cu, xn, R, rs, si, pw);
-      dot = 0;
-      for (int a = 0; a < 7; a++) dot += R[a] * R[a];
-      nR = sqrt(dot);
+      ttrate = formR(cu, xn, R);
+      dot = norm2<7>(R);
       if (0.5 * dot <= ls1 + ls2 * alpha || ls > 10) {
         for (int a = 0; a < 7; a++) x[a] = xn[a];
         break;
@@ -1134,9 +1165,9 @@ __device__ void voxel_update(const StressArgs& a, long long v, bool valid, int& 
   if (iter0 || no_load) {
     for (int i = 0; i < 36; i++) cep[i] = __ldg(rec->C + i);
     if (!no_load) {
-      double rs[NS], si[NS], pw[NS], R1[6];
-      slips(s, stress, tt, rs, si, pw);
-      formR1(s, stress, rs, si, R1);
+      double R1[6];
+      slips(s, stress, tt);
+      formR1(s, stress, R1);
       for (int i = 0; i < 6; i++) stress[i] -= R1[i];
     }
     ttrate = 0.0;
@@ -1209,11 +1240,14 @@ __device__ void voxel_update(const StressArgs& a, long long v, bool valid, int& 
     ok = !(fail || isnan(tt) || anynan(stress, 6));
     if (ok) {
       // mm10_tangent for Voce (JA = JB = 0): T = (J11 - J12 J21 / J22)^-1 C, symmetrised
-      double JJ[36];
+      double JJ[36], J2[6];
+      const double i22 = 1.0 / Jl[48];
+      for (int j = 0; j < 6; j++) J2[j] = Jl[42 + j] * i22;
       for (int i = 0; i < 6; i++)
-        for (int j = 0; j < 6; j++) JJ[6 * i + j] = Jl[7 * i + j] - Jl[7 * i + 6] * (Jl[42 + j] / Jl[48]);
+        for (int j = 0; j < 6; j++) JJ[6 * i + j] = Jl[7 * i + j] - Jl[7 * i + 6] * J2[j];
       // LU of JJ once, 6 right-hand sides (columns of C)
       int piv[6];
+      double inv[6];
       for (int k = 0; k < 6; k++) {
         int p = k;
         double best = fabs(JJ[6 * k + k]);
@@ -1222,9 +1256,9 @@ __device__ void voxel_update(const StressArgs& a, long long v, bool valid, int& 
         piv[k] = p;
         if (p != k)
           for (int j = 0; j < 6; j++) { double t = JJ[6 * k + j]; JJ[6 * k + j] = JJ[6 * p + j]; JJ[6 * p + j] = t; }
-        double inv = 1.0 / JJ[6 * k + k];
+        inv[k] = 1.0 / JJ[6 * k + k];
         for (int i = k + 1; i < 6; i++) {
-          double l = JJ[6 * i + k] * inv;
+          double l = JJ[6 * i + k] * inv[k];
           JJ[6 * i + k] = l;
           for (int j = k + 1; j < 6; j++) JJ[6 * i + j] -= l * JJ[6 * k + j];
         }
@@ -1244,7 +1278,7 @@ __device__ void voxel_update(const StressArgs& a, long long v, bool valid, int& 
         for (int i = 5; i >= 0; i--) {
           double sacc = b[i];
           for (int k = i + 1; k < 6; k++) sacc -= JJ[6 * i + k] * b[k];
-          b[i] = sacc / JJ[6 * i + i];
+          b[i] = sacc * inv[i];
         }
         for (int i = 0; i < 6; i++) T[6 * i + c] = b[i];
       }
@@ -1276,14 +1310,14 @@ __device__ void voxel_update(const StressArgs& a, long long v, bool valid, int& 
     for (int i = 0; i < 3; i++)
       for (int j = 0; j < 3; j++) tr[3 * i + j] = nRp[3 * j + i];
     rt2rvw(tr, RW);
-    double rs[NS], si[NS], pw[NS], wb[3] = {0, 0, 0};
-    slips(s, stress, tt, rs, si, pw);
+    // the slips at (stress, tt) are the last residual's
+    double wb[3] = {0, 0, 0};
     double tid = s.tinc * cr->iD_v;
     for (int i = 0; i < NS; i++) {
       double q0[3], qs[3];
       for (int k = 0; k < 3; k++) q0[k] = __ldg(rec->qs + 3 * i + k);
       for (int k = 0; k < 3; k++) qs[k] = RW[3 * k] * q0[0] + RW[3 * k + 1] * q0[1] + RW[3 * k + 2] * q0[2];
-      double f = si[i] + rs[i] * tid;
+      double f = s.si[i] + s.rs[i] * tid;
       for (int k = 0; k < 3; k++) wb[k] += f * qs[k];
     }
     double W[9] = {0.0, wb[2], wb[1], -wb[2], 0.0, wb[0], -wb[1], -wb[0], 0.0};
