@@ -1320,7 +1320,10 @@ int stress(Ctx* c, int step, int iter, long long* local_iters, int* fails,
   a.cost = nullptr;
   a.qchunk = c->qchunk;
   a.qbps = c->qbps;
-  if (c->sched == CPFFT_SCHED_QUEUE && iter > 0 && c->n_crys_vox) {
+  const bool density = c->h_type == 7 || c->h_type == 4;  // their solve has no voxel queue
+  if (c->sched == CPFFT_SCHED_QUEUE && iter > 0 && c->n_crys_vox && density) {
+    c->qtuned = true;
+  } else if (c->sched == CPFFT_SCHED_QUEUE && iter > 0 && c->n_crys_vox) {
     a.perm = c->vperm;
     a.queue = c->vq + 128;
     a.cost = c->vcost;

@@ -40,7 +40,6 @@ namespace {
 
 constexpr int NS = CPFFT_NSLIP;  // slip systems
 constexpr bool MTS = CPFFT_LAW == 2;
-constexpr bool MRR = CPFFT_LAW == 7 || CPFFT_LAW == 4;  // the dislocation-density laws
 // the temperature of the reference's FFT path (drive_10_update, src/rstgp1.f:832)
 constexpr double TEMP = 297.0;
 
@@ -965,15 +964,11 @@ __global__ void __launch_bounds__(128) stress_kernel(StressArgs a) {
     const bool mine = valid && (!a.mises || __ldg(a.mises + v) < 0);
     int it = 0, pit = 0, rj = 0;
     bool ok = true;
-#if CPFFT_LAW == 7 || CPFFT_LAW == 4
-    if (mine) voxel_update_mrr(a, v, it, pit, ok);  // no learned guess for these grids
-#else
     if (WARM) {
       voxel_update<true>(a, v, mine, it, pit, ok, rj, &gb);
     } else if (mine) {
       voxel_update<false>(a, v, true, it, pit, ok, rj, nullptr);
     }
-#endif
     if (mine) {
       iters += it;
       piters += pit;
@@ -1618,9 +1613,27 @@ cudaError_t launch_mises(const StressArgs& a, cudaStream_t s) {
 }
 #endif
 
-cudaError_t CPFFT_STRESS_LAUNCH(const StressArgs& a, bool warm_in, cudaStream_t s) {
+#if CPFFT_LAW == 7 || CPFFT_LAW == 4
+// The dislocation-density laws: no learned guess, no alternative starts and no voxel queue
+// (the solve's warps hold two voxels and are dealt over a persistent grid).
+cudaError_t CPFFT_STRESS_LAUNCH(const StressArgs& a, bool, cudaStream_t s) {
   if (a.N3 <= 0) return cudaSuccess;
-  const bool warm = warm_in && !MRR;  // the MRR solve has no learned guess
+  int dev = 0, sms = 0, per = 0;
+  cudaError_t e;
+  if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
+  if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, mrr_solve, MRR_NT, 0)) != cudaSuccess) return e;
+  const unsigned blocks = (unsigned)((a.N3 + 127) / 128);
+  const unsigned groups = (unsigned)((a.N3 + MRR_VB - 1) / MRR_VB);
+  mrr_pre<<<blocks, 128, 0, s>>>(a);
+  mrr_solve<<<std::min((unsigned)(sms * std::max(per, 1)), groups), MRR_NT, 0, s>>>(a);
+  mrr_post<<<blocks, 128, 0, s>>>(a);
+  g_kernel_launches += 3;
+  return cudaGetLastError();
+}
+#else
+cudaError_t CPFFT_STRESS_LAUNCH(const StressArgs& a, bool warm, cudaStream_t s) {
+  if (a.N3 <= 0) return cudaSuccess;
   if (warm) {  // set on every call: the attribute belongs to the current device
     cudaError_t e = cudaFuncSetAttribute(stress_kernel<true>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -1646,6 +1659,7 @@ cudaError_t CPFFT_STRESS_LAUNCH(const StressArgs& a, bool warm_in, cudaStream_t 
   g_kernel_launches += 1;
   return cudaGetLastError();
 }
+#endif
 
 #if CPFFT_FIRST_UNIT
 cudaError_t launch_voxel_queue(const unsigned char* cost, long long N3, unsigned int* scratch,
