@@ -182,6 +182,11 @@ SIGNATURES = {
 MLP_NIN, MLP_NOUT, MLP_PARAMS, MLP_NORM = 20, 7, 22800, 54
 
 
+_new_bytes = ctypes.pythonapi.PyBytes_FromStringAndSize
+_new_bytes.restype = ctypes.py_object
+_new_bytes.argtypes = [ctypes.c_char_p, ctypes.c_ssize_t]
+
+
 def _fp(a):
     if a is None:
         return None
@@ -381,8 +386,8 @@ class Solver:
 
     # --- mirror of the reference routines ------------------------------------------
     def drive_eps_sig(self, step, it, Fn=None, Fn1=None, want_P=True, want_K4=False):
-        P = np.zeros((9, self.N3)) if want_P else None
-        K = np.zeros((81, self.N3)) if want_K4 else None
+        P = np.empty((9, self.N3)) if want_P else None
+        K = np.empty((81, self.N3)) if want_K4 else None
         rc = _check(load_library().cpfft_stress_update(step, it, _dp(Fn), _dp(Fn1), _dp(P),
                                                        _dp(K)), "drive_eps_sig")
         return P, K, rc
@@ -396,7 +401,7 @@ class Solver:
                 "starts_dropped": c[3], "substepped": c[4]}
 
     def G_K_dF(self, x, flgK=True):
-        y = np.zeros((9, self.N3))
+        y = np.empty((9, self.N3))
         _check(load_library().cpfft_green_apply(_dp(np.ascontiguousarray(x)), _dp(y),
                                                 int(flgK)), "G_K_dF")
         return y
@@ -404,13 +409,13 @@ class Solver:
     def G_K_dF_f32(self, x, flgK=True):
         """The FP32 operator of the mixed-precision Krylov iterations."""
         x = np.ascontiguousarray(x, np.float32)
-        y = np.zeros((9, self.N3), np.float32)
+        y = np.empty((9, self.N3), np.float32)
         _check(load_library().cpfft_green_apply_f32(_fp(x), _fp(y), int(flgK)), "G_K_dF_f32")
         return y
 
     def G_K_dF_df(self, x, flgK=True):
         """The double-float FP64-accurate operator of the mixed-precision solver."""
-        y = np.zeros((9, self.N3))
+        y = np.empty((9, self.N3))
         _check(load_library().cpfft_green_apply_df(_dp(np.ascontiguousarray(x)), _dp(y),
                                                    int(flgK)), "G_K_dF_df")
         return y
@@ -419,7 +424,7 @@ class Solver:
         _check(load_library().cpfft_set_K4(_dp(np.ascontiguousarray(K4))), "set_K4")
 
     def fftPcg(self, b, tol):
-        x = np.zeros((9, self.N3))
+        x = np.empty((9, self.N3))
         its = ctypes.c_int(0)
         rc = load_library().cpfft_cg(_dp(np.ascontiguousarray(b)), _dp(x), tol,
                                      ctypes.byref(its))
@@ -445,9 +450,9 @@ class Solver:
         return rc, Pbar, st.as_dict()
 
     def fields(self, history=False):
-        F = np.zeros((9, self.N3))
-        P = np.zeros((9, self.N3))
-        H = np.zeros((_check(load_library().cpfft_hist_words(), "cpfft_hist_words"), self.N3)) \
+        F = np.empty((9, self.N3))
+        P = np.empty((9, self.N3))
+        H = np.empty((_check(load_library().cpfft_hist_words(), "cpfft_hist_words"), self.N3)) \
             if history else None
         _check(load_library().cpfft_sync_to_host(_dp(F), _dp(P), _dp(H)), "sync_to_host")
         return (F, P, H) if history else (F, P)
@@ -458,9 +463,10 @@ class Solver:
         L = load_library()
         n = ctypes.c_longlong(0)
         L.cpfft_format_flat(int(quantity), None, 0, ctypes.byref(n))
-        buf = ctypes.create_string_buffer(n.value)
-        _check(L.cpfft_format_flat(int(quantity), buf, n.value, ctypes.byref(n)), "format_flat")
-        return buf.raw[:n.value]
+        # the text is written straight into the (new, not yet shared) bytes object
+        out = _new_bytes(None, n.value)
+        _check(L.cpfft_format_flat(int(quantity), out, n.value, ctypes.byref(n)), "format_flat")
+        return out
 
     def write_flat(self, quantity, step, structure_name="cpfft", directory=""):
         _check(load_library().cpfft_write_flat(int(quantity), int(step),
@@ -469,7 +475,7 @@ class Solver:
 
     def f2disp(self, lengths=(100.0, 100.0, 100.0)):
         """Nodal displacements (the reference's u array as ((N+1)^3, 3))."""
-        u = np.zeros(3 * (self.N + 1) ** 3)
+        u = np.empty(3 * (self.N + 1) ** 3)
         _check(load_library().cpfft_f2disp(float(lengths[0]), float(lengths[1]),
                                            float(lengths[2]), _dp(u)), "f2disp")
         return u.reshape(-1, 3)

@@ -1,6 +1,9 @@
 // api.cu -- the C-ABI of include/cpfft_gpu.h: device context, material set-up, and the
 // host-side control of the resident Newton-Krylov loop (FFT_nr3 / fftPcg /
 // tangent_homo / NBC_update of src/FFT_nr3.f and src/tangent_homo.f).
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -23,7 +26,7 @@
 // element result text (results.cu)
 void host_e15(double v, char* out);
 cudaError_t launch_format_flat(const double* hist, long long N3, int word0, int nvals, char* text,
-                               unsigned char* flags, cudaStream_t st);
+                               unsigned char* flags, int* any, cudaStream_t st);
 cudaError_t launch_format_values(const double* x, long long n, char* out, unsigned char* flags,
                                  cudaStream_t st);
 
@@ -455,6 +458,9 @@ struct Ctx {
   OriRec* oris = nullptr;
   CrysRec* cryss = nullptr;
   PowTab* ptabs = nullptr;  // the crystals' power tables
+  double* dct_tab = nullptr;  // f2disp's cosine table, (N + 1)^2 (first call)
+  char* fmt_buf = nullptr;    // result-text buffer, kept up to FMT_KEEP bytes
+  long long fmt_cap = 0;
   // materials: 0-based material of every voxel; per material 0 = crystal, 1 = mm01
   // (cpfft_set_mises), 2 = declared non-crystal and not yet defined
   std::vector<int> mat;
@@ -549,6 +555,38 @@ void kt_reset(Ctx* c) {
 }
 thread_local Ctx* g_ctx = nullptr;
 
+// Pages of large host output buffers made present by helper threads while the GPU works: a
+// device-to-host copy into untouched pages faults them one by one (151 MB: 5.5 ms against
+// 0.8 ms into present pages; two to four threads prepare them in 1.8 ms).  Contents are
+// kept; a buffer the call cannot prepare is left to the copy.
+class Prefault {
+  std::vector<std::thread> th_;
+
+ public:
+  Prefault(std::initializer_list<std::pair<void*, size_t>> bufs) {
+    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+    for (const auto& b : bufs) {
+      const size_t a0 = ((size_t)b.first + page - 1) / page * page;
+      const size_t a1 = ((size_t)b.first + b.second) / page * page;
+      if (!b.first || b.second < (4u << 20) || a1 <= a0) continue;
+      const size_t nt = std::min<size_t>(4, (a1 - a0) >> 22), part = (a1 - a0) / (nt * page) * page;
+      for (size_t k = 0; k < nt && part; k++) {
+        const size_t p0 = a0 + k * part, p1 = k + 1 == nt ? a1 : p0 + part;
+        try {
+          th_.emplace_back([p0, p1] { madvise((void*)p0, p1 - p0, 23 /* MADV_POPULATE_WRITE */); });
+        } catch (...) {  // no thread to be had: the copy faults the pages itself
+          return;
+        }
+      }
+    }
+  }
+  void join() {
+    for (auto& t : th_) t.join();
+    th_.clear();
+  }
+  ~Prefault() { join(); }
+};
+
 #define TRY(expr)                 \
   do {                            \
     int _rc = (expr);             \
@@ -573,7 +611,7 @@ void free_ctx(Ctx* c) {
                   c->hist[0], c->hist[1], c->K4f, c->xf, c->rf, c->pf, c->Apf, c->ori, c->crys,
                   c->oris, c->cryss, c->S, c->Sf, c->tw, c->twf, c->part, c->sc, c->stats,
                   c->k0sum, c->K4lo, c->twdf, c->vcost, c->vperm, c->vq, c->pre_dev,
-                  c->mises, c->misess, c->bar, c->ptabs};
+                  c->mises, c->misess, c->bar, c->ptabs, c->dct_tab, c->fmt_buf};
   for (void* q : ptrs)
     if (q) cudaFree(q);
   if (c->h_sc) cudaFreeHost(c->h_sc);
@@ -2117,7 +2155,9 @@ int cpfft_stress_update(int step, int iter, const double* Fn, const double* Fn1,
   TRY(cpfft_set_F(Fn, Fn1));
   long long li;
   int fails;
+  Prefault pf({{Pn1, 9 * c->N3 * sizeof(double)}, {K4, 81 * c->N3 * sizeof(double)}});
   TRY(stress(c, step, iter, &li, &fails));
+  pf.join();
   if (Pn1) CK(cudaMemcpyAsync(Pn1, c->P, 9 * c->N3 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   if (K4) CK(cudaMemcpyAsync(K4, c->K4, 81 * c->N3 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
   TRY(sync(c));
@@ -2163,8 +2203,10 @@ int cpfft_green_apply(const double* x, double* y, int flgK) {
   TRY(need_ctx());
   Ctx* c = g_ctx;
   const size_t f9 = 9 * c->N3 * sizeof(double);
+  Prefault pf({{y, f9}});
   CK(cudaMemcpyAsync(c->io, x, f9, cudaMemcpyHostToDevice, c->st));
   TRY(matvec64(c, c->io, c->b, flgK ? 1 : 0));
+  pf.join();
   CK(cudaMemcpyAsync(y, c->b, f9, cudaMemcpyDeviceToHost, c->st));
   return sync(c);
 }
@@ -2178,10 +2220,12 @@ int cpfft_green_apply_f32(const float* x, float* y, int flgK) {
     return CPFFT_ERR_BAD_ARG;
   }
   const size_t f9 = 9 * c->N3 * sizeof(float);
+  Prefault pf({{y, f9}});
   CK(cudaMemcpyAsync(c->rf, x, f9, cudaMemcpyHostToDevice, c->st));
   c->f32_matvecs++;
   TRY(cuda_check(green_apply<float>(c->rf, c->K4f, flgK ? 1 : 0, c->Apf, c->Sf, c->twf, c->g, c->st),
                  "green_apply fp32"));
+  pf.join();
   CK(cudaMemcpyAsync(y, c->Apf, f9, cudaMemcpyDeviceToHost, c->st));
   return sync(c);
 }
@@ -2195,8 +2239,10 @@ int cpfft_green_apply_df(const double* x, double* y, int flgK) {
     return CPFFT_ERR_BAD_ARG;
   }
   const size_t f9 = 9 * c->N3 * sizeof(double);
+  Prefault pf({{y, f9}});
   CK(cudaMemcpyAsync(c->io, x, f9, cudaMemcpyHostToDevice, c->st));
   TRY(matvec_acc(c, c->io, c->b, flgK ? 1 : 0));
+  pf.join();
   CK(cudaMemcpyAsync(y, c->b, f9, cudaMemcpyDeviceToHost, c->st));
   return sync(c);
 }
@@ -2207,8 +2253,10 @@ int cpfft_cg(const double* b, double* x, double tol, int* iters) {
   c->cg_rel_only = false;
   const size_t f9 = 9 * c->N3 * sizeof(double);
   int its = 0;
+  Prefault pf({{x, f9}});
   CK(cudaMemcpyAsync(c->b, b, f9, cudaMemcpyHostToDevice, c->st));
   int rc = cg(c, c->b, c->io, tol, &its);
+  pf.join();
   if (iters) *iters = its;
   if (rc < 0 && rc != CPFFT_ERR_CG_MAXIT) return rc;
   CK(cudaMemcpyAsync(x, c->io, f9, cudaMemcpyDeviceToHost, c->st));
@@ -2784,24 +2832,43 @@ int cpfft_format_flat(int quantity, char* text, long long capacity, long long* l
     cpfft_set_error("cpfft_format_flat: buffer of %lld bytes needed", total);
     return CPFFT_ERR_BAD_ARG;
   }
-  char* dt = nullptr;
-  unsigned char* dfl = nullptr;
-  int rc = 0;
-  if ((rc = dalloc(dt, total)) || (rc = dalloc(dfl, 6 * c->N3))) {
-    cudaFree(dt);
-    cudaFree(dfl);
-    return rc;
+  // text, flags of the fields left to the host, and whether there are any; the buffer stays
+  // with the context while it is small
+  constexpr long long FMT_KEEP = 64LL << 20;
+  const long long off_fl = (total + 15) & ~15LL, off_any = (off_fl + 6 * c->N3 + 15) & ~15LL;
+  const long long need = off_any + 16;
+  char* dt = c->fmt_buf;
+  if (need > c->fmt_cap) {
+    if (c->fmt_buf) cudaFree(c->fmt_buf);
+    c->fmt_buf = nullptr;
+    c->fmt_cap = 0;
+    TRY(dalloc(dt, need));
+    if (need <= FMT_KEEP) {
+      c->fmt_buf = dt;
+      c->fmt_cap = need;
+    }
   }
-  std::vector<unsigned char> fl(6 * c->N3);
+  unsigned char* dfl = (unsigned char*)dt + off_fl;
+  int any = 0, rc = 0;
+  std::vector<unsigned char> fl;
   cudaError_t e;
-  if ((e = launch_format_flat(c->hist[c->hn], c->N3, word0, nvals, dt, dfl, c->st)) ||
-      (e = cudaMemcpyAsync(text, dt, total, cudaMemcpyDeviceToHost, c->st)) ||
-      (e = cudaMemcpyAsync(fl.data(), dfl, 6 * c->N3, cudaMemcpyDeviceToHost, c->st)) ||
-      (e = cudaStreamSynchronize(c->st)))
+  {
+    Prefault pf({{text, (size_t)total}});
+    if ((e = launch_format_flat(c->hist[c->hn], c->N3, word0, nvals, dt, dfl, (int*)(dt + off_any), c->st)))
+      rc = cuda_check(e, "cpfft_format_flat");
+  }
+  if (!rc && ((e = cudaMemcpyAsync(text, dt, total, cudaMemcpyDeviceToHost, c->st)) ||
+              (e = cudaMemcpyAsync(&any, dt + off_any, sizeof(int), cudaMemcpyDeviceToHost, c->st)) ||
+              (e = cudaStreamSynchronize(c->st))))
     rc = cuda_check(e, "cpfft_format_flat");
-  cudaFree(dt);
-  cudaFree(dfl);
-  if (rc) return rc;
+  if (!rc && any) {
+    fl.resize(6 * c->N3);
+    if ((e = cudaMemcpyAsync(fl.data(), dfl, 6 * c->N3, cudaMemcpyDeviceToHost, c->st)) ||
+        (e = cudaStreamSynchronize(c->st)))
+      rc = cuda_check(e, "cpfft_format_flat");
+  }
+  if (dt != c->fmt_buf) cudaFree(dt);
+  if (rc || !any) return rc;
   // the fields the device could not round exactly: formatted here from the same values
   std::vector<double> hv;
   for (long long v = 0; v < c->N3; v++)
@@ -2870,29 +2937,34 @@ int cpfft_f2disp(double lx, double ly, double lz, double* u) {
   }
   const int N = c->N;
   const long long N1 = N + 1, nodes = N1 * N1 * N1;
-  // cos(pi k i / N) with the angle reduced to [0, 2 pi) in integers first
-  std::vector<double> ctab(N1 * N1);
-  for (long long k = 0; k < N1; k++)
-    for (long long i = 0; i < N1; i++) {
-      const long long m = (k * i) % (2LL * N);
-      ctab[k * N1 + i] = (double)cosl(3.14159265358979323846264338327950288L * m / N);
-    }
-  double *dtab = nullptr, *work = nullptr, *du = nullptr;
-  int rc = 0;
-  if ((rc = dalloc(dtab, ctab.size() * sizeof(double))) ||
-      (rc = dalloc(work, 6 * nodes * sizeof(double))) || (rc = dalloc(du, 3 * nodes * sizeof(double)))) {
-    cudaFree(dtab); cudaFree(work); cudaFree(du);
-    return rc;
+  if (!c->dct_tab) {  // cos(pi k i / N), from the N + 1 distinct values; kept by the context
+    std::vector<double> cv(N1), ctab(N1 * N1);
+    for (long long m = 0; m < N1; m++) cv[m] = (double)cosl(3.14159265358979323846264338327950288L * m / N);
+    for (long long k = 0; k < N1; k++)
+      for (long long i = 0; i < N1; i++) {
+        const long long m = (k * i) % (2LL * N);
+        ctab[k * N1 + i] = cv[m <= N ? m : 2LL * N - m];
+      }
+    TRY(dalloc(c->dct_tab, ctab.size() * sizeof(double)));
+    CK(cudaMemcpyAsync(c->dct_tab, ctab.data(), ctab.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
+    TRY(sync(c));
   }
+  // scratch: the CG's fields, which hold nothing between calls (a nodal field has
+  // 3 (N + 1)^3 <= 9 N^3 values from N = 3 on)
+  double *work = c->r, *du = c->p, *small = nullptr;
+  if (3 * nodes > 9 * c->N3) {
+    TRY(dalloc(small, 6 * nodes * sizeof(double)));
+    work = small;
+    du = small + 3 * nodes;
+  }
+  int rc = 0;
   cudaError_t e;
-  if ((e = cudaMemcpyAsync(dtab, ctab.data(), ctab.size() * sizeof(double), cudaMemcpyHostToDevice, c->st)) ||
-      (e = f2disp_device(c->Fn1, N, lx, ly, lz, dtab, work, du, c->st)) ||
-      (e = cudaMemcpyAsync(u, du, 3 * nodes * sizeof(double), cudaMemcpyDeviceToHost, c->st)) ||
+  Prefault pf({{u, 3 * nodes * sizeof(double)}});
+  if ((e = f2disp_device(c->Fn1, N, lx, ly, lz, c->dct_tab, work, du, c->st)) ||
+      (pf.join(), e = cudaMemcpyAsync(u, du, 3 * nodes * sizeof(double), cudaMemcpyDeviceToHost, c->st)) ||
       (e = cudaStreamSynchronize(c->st)))
     rc = cuda_check(e, "cpfft_f2disp");
-  cudaFree(dtab);
-  cudaFree(work);
-  cudaFree(du);
+  if (small) cudaFree(small);
   return rc;
 }
 
