@@ -650,6 +650,12 @@ int read_scalar(Ctx* c, int slot, double* out) {
   return 0;
 }
 
+// all scalars to the host, one wait
+int read_scalars(Ctx* c) {
+  CK(cudaMemcpyAsync(c->h_sc, c->sc, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  return sync(c);
+}
+
 int dnrm2(Ctx* c, const double* x, double* out) {
   CK(dev_dot(x, x, 9 * c->N3, c->part, c->sc, SC_TMP, OP_STORE, c->st));
   double v;
@@ -829,8 +835,7 @@ int cg64_small(Ctx* c, const double* b, double* x, double tol, int* iters) {
   CK(cg_small_solve(b, x, c->r, c->p, c->w, c->Ap, c->K4, c->S, c->tw, c->g, tol, maxIter, c->part,
                     c->sc, c->bar, c->st));
   TRY(kt_stop(c));
-  CK(cudaMemcpyAsync(c->h_sc, c->sc, SC_COUNT * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  TRY(sync(c));
+  TRY(read_scalars(c));
   const int stop = (int)c->h_sc[SC_STOP], it = (int)c->h_sc[SC_CNT];
   if (stop == STOP_BARRIER) {
     cpfft_set_error("CG: a grid barrier ran out of its wait");
@@ -993,7 +998,7 @@ int cg_mixed(Ctx* c, const double* b, double* x, double tol, int* iters, bool us
 
 // One preconditioned FP32 CG iteration on the device: p = r + beta p (and rr <- rr_new),
 // Ap = G0(K4f : p) with pAp = <K4f : p, p> and alpha = rr / pAp, x += alpha p, r -= alpha Ap
-// with rr_new = <r, r>_K0 and beta, then the stop test (k_cg_cond).  `timed` brackets the
+// with rr_new = <r, r>_K0 and beta, then the stop test (cg_cond).  `timed` brackets the
 // Green apply with the per-launch CUDA events (never inside a capture).
 int cg_pre_body(Ctx* c, bool use_handle, bool timed) {
   const long long n = 9 * c->N3;
@@ -1005,27 +1010,26 @@ int cg_pre_body(Ctx* c, bool use_handle, bool timed) {
     // updated in the first, x, r and the partials of <r, r>_K0 in the last
     if (timed) kt_start(c, KT_G32);
     CK(green_cg_iteration(c->xf, c->rf, c->pf, c->K4f, c->Sf, c->twf, g, c->st, c->part,
-                          c->part, c->pre_dev + 36, c->sc));
+                          c->part, c->pre_dev + 36, c->sc, c->cg_handle, use_handle));
     if (timed) TRY(kt_stop(c));
-    CK(dev_final(c->part, (c->N / 2) * c->N, c->sc, SC_RRNEW, OP_BETA, c->st));
-    CK(dev_cg_cond(c->sc, c->cg_handle, use_handle, c->st));
     return 0;
   }
   CK(dev_cg_p<float>(c->pf, c->rf, n, c->sc, c->st));
   if (timed) kt_start(c, KT_G32);
-  CK(green_apply_dot<float>(c->pf, c->K4f, 1, c->Apf, c->Sf, c->twf, g, c->st, c->part, &np));
+  CK(green_apply_dot<float>(c->pf, c->K4f, 1, c->Apf, c->Sf, c->twf, g, c->st, c->part, &np, nullptr,
+                            c->sc));
   if (timed) TRY(kt_stop(c));
   if (!np) {
     cpfft_set_error("internal: the preconditioned product was not fused");
     return CPFFT_ERR_CUDA;
   }
-  CK(dev_final(c->part, np, c->sc, SC_PAP, OP_ALPHA, c->st));
-  CK(dev_cg_xr_k0(c->xf, c->rf, c->pf, c->Apf, c->N3, c->pre_dev + 36, c->part, c->sc, c->st));
-  CK(dev_cg_cond(c->sc, c->cg_handle, use_handle, c->st));
+  if (np > 0) CK(dev_final(c->part, np, c->sc, SC_PAP, OP_ALPHA, c->st));
+  CK(dev_cg_xr_k0(c->xf, c->rf, c->pf, c->Apf, c->N3, c->pre_dev + 36, c->part, c->sc, c->cg_handle,
+                  use_handle, c->st));
   return 0;
 }
 
-// Capture the iteration once into a graph whose WHILE node repeats it while k_cg_cond
+// Capture the iteration once into a graph whose WHILE node repeats it while cg_cond
 // says so (the node's default value runs the body at least once per launch).  Every
 // buffer and launch shape is fixed for the context; alpha, beta and the stop test's
 // inputs live in device memory.  If anything fails, the iterations run eagerly instead.
@@ -1087,27 +1091,19 @@ void build_cg_graph(Ctx* c) {
   c->cg_graph_state = 1;
 }
 
-// Run iterations from the current (rf, pf, xf) until k_cg_cond stops them: the first one
-// eagerly with the Green apply timed (the per-launch figure of the FP32 operator), the
-// rest as one launch of the iteration graph.  rr (in) is <r,r>_K0 now; *rr_out the value
-// at the end; *it_out the iteration count after the segment; *stop the reason.
-int cg_segment(Ctx* c, double rr, double rn, double tolb, double tol, double delta, int it,
-               int maxIter, double beta, double* rr_out, double* rr_prev_out, int* it_out,
-               int* stop) {
-  double* h = c->h_sc;
-  h[SC_BETA] = beta;
-  h[SC_RRNEW] = rr;
-  CK(cudaMemcpyAsync(c->sc + SC_BETA, h + SC_BETA, sizeof(double), cudaMemcpyHostToDevice, c->st));
-  CK(cudaMemcpyAsync(c->sc + SC_RRNEW, h + SC_RRNEW, sizeof(double), cudaMemcpyHostToDevice, c->st));
-  h[SC_RR0] = rr; h[SC_RN] = rn; h[SC_TOLB] = tolb; h[SC_TOL] = tol; h[SC_DELTA] = delta;
-  h[SC_CNT] = (double)it; h[SC_MAXIT] = (double)maxIter; h[SC_STOP] = 0.0;
-  CK(cudaMemcpyAsync(c->sc + SC_RR0, h + SC_RR0, (SC_STOP - SC_RR0 + 1) * sizeof(double),
-                     cudaMemcpyHostToDevice, c->st));
+// Enqueue iterations from the current (rf, pf, xf) and the <r,r>_K0 in sc[SC_RRNEW] until
+// cg_cond stops them: the first one eagerly with the Green apply timed (the per-launch figure
+// of the FP32 operator), the rest as one launch of the iteration graph.  rn: the true residual
+// norm now; rrk2: the denominator of the first beta (0: beta is 0).  *done: the eager iterations.
+// The results are read with the caller's next transfer of the scalars (cg_segment_end).
+int cg_segment(Ctx* c, double rn, double tolb, double tol, double delta, int it, int maxIter,
+               double rrk2, int* done) {
+  CK(dev_cg_start(c->sc, rn, tolb, tol, delta, it, maxIter, rrk2, c->st));
   build_cg_graph(c);
-  int done = 0;
+  *done = 0;
   for (;;) {
-    TRY(cg_pre_body(c, false, done == 0));
-    done++;
+    TRY(cg_pre_body(c, false, *done == 0));
+    ++*done;
     if (c->cg_graph_state == 1) {  // the graph's gate skips its loop if already stopped
       kt_start(c, KT_CGGRAPH);
       CK(cudaGraphLaunch(c->cg_exec, c->st));
@@ -1119,17 +1115,25 @@ int cg_segment(Ctx* c, double rr, double rn, double tolb, double tol, double del
     TRY(read_scalar(c, SC_STOP, &st));
     if (st != 0.0) break;
   }
-  CK(cudaMemcpyAsync(h + SC_CNT, c->sc + SC_CNT, (SC_STOP - SC_CNT + 1) * sizeof(double),
-                     cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(h + SC_RR, c->sc + SC_RR, sizeof(double), cudaMemcpyDeviceToHost, c->st));
-  TRY(read_scalar(c, SC_RRNEW, rr_out));
-  *rr_prev_out = h[SC_RR];  // <r,r>_K0 before the last iteration (its beta's denominator)
+  return 0;
+}
+
+// The segment's results from the scalars in h_sc (copied and waited for): *it (in: the count
+// at its start) the iteration count, *rr_prev <r,r>_K0 before the last iteration (its beta's
+// denominator), *stop the reason it ended.
+int cg_segment_end(Ctx* c, int done, int* it, double* rr_prev, int* stop) {
+  const double* h = c->h_sc;
   const int it_end = (int)h[SC_CNT];
-  const long long its = it_end - it;
+  const long long its = it_end - *it;
   c->f32_matvecs += its;
   if (c->cg_graph_state == 1) g_kernel_launches += (its - done) * c->cg_body_launches;
-  *it_out = it_end;
+  *it = it_end;
+  *rr_prev = h[SC_RR];
   *stop = (int)h[SC_STOP];
+  if (*stop == STOP_NONFINITE) {
+    cpfft_set_error("FP32 CG residual is not finite");
+    return CPFFT_ERR_NONFINITE;
+  }
   return 0;
 }
 
@@ -1176,43 +1180,37 @@ int cg_mixed_pre(Ctx* c, const double* b, double* x, double tol, int* iters, boo
   CK(cudaMemsetAsync(c->xf, 0, n * sizeof(float), c->st));
   CK(cudaMemcpyAsync(c->pf, c->rf, n * sizeof(float), cudaMemcpyDeviceToDevice, c->st));
   CK(dev_dot_k0(c->rf, c->rf, c->N3, c->pre_dev + 36, c->part, c->sc, SC_RRNEW, OP_STORE, c->st));
-  double rr;
-  TRY(read_scalar(c, SC_RRNEW, &rr));
-  double beta = 0.0;  // the first iteration's p = r + 0 p = r
+  double rrk2 = 0.0;  // the first iteration's p = r + 0 p = r
   int it = 0, restarts = 0;
   bool converged = false;
   for (;;) {
     // one segment of iterations on the device: until <r,r>_K0 has dropped by delta, the
-    // true residual it predicts meets the stop test, or maxIter
-    int stop = 0;
-    double rr_prev = rr;
-    TRY(cg_segment(c, rr, rn, tolb, tola, delta, it, maxIter, beta, &rr, &rr_prev, &it, &stop));
-    if (stop == STOP_NONFINITE) { cpfft_set_error("FP32 CG residual is not finite"); return CPFFT_ERR_NONFINITE; }
-    // reliable update: x += G(xf / scale) in FP64-accurate arithmetic, true residual
+    // true residual it predicts meets the stop test, or maxIter; then the reliable update,
+    // x += G(xf / scale) in FP64-accurate arithmetic and the true residual, enqueued behind it:
+    // the host waits once for both
+    int stop = 0, done = 0;
+    TRY(cg_segment(c, rn, tolb, tola, delta, it, maxIter, rrk2, &done));
     restarts++;
-    CK(cudaMemsetAsync(c->w2, 0, n * sizeof(double), c->st));
-    CK(dev_add_f32(c->w2, c->xf, 1.0 / scale, n, c->st));
+    CK(dev_take_f32(c->w2, c->xf, 1.0 / scale, n, c->st));
     TRY(matvec_acc(c, c->w2, c->Ap, 0));
     CK(dev_axpy(x, c->Ap, 1.0, n, c->st));
     TRY(matvec_acc(c, x, c->Ap, 1));
-    CK(dev_sub(c->w, b, c->Ap, n, c->st));
-    TRY(dnrm2(c, c->w, &rn));
+    CK(dev_sub_norm(c->w, b, c->Ap, n, c->part, c->sc, SC_TMP, c->st));
+    TRY(read_scalars(c));
+    double rr_prev;
+    TRY(cg_segment_end(c, done, &it, &rr_prev, &stop));
+    rn = std::sqrt(c->h_sc[SC_TMP]);
     if (!std::isfinite(rn)) { cpfft_set_error("FP64 residual is not finite"); return CPFFT_ERR_NONFINITE; }
     if (rn <= tolb || rn <= tola) { converged = true; break; }
     if (it >= maxIter) break;
     // restart from G0 of the true residual, keeping the search direction (rescaled)
     const double nscale = 1.0 / rn, k = nscale / scale;
-    CK(dev_to_f32(c->Apf, c->w, nscale, n, c->st));
+    CK(dev_restart_f32(c->Apf, c->w, nscale, c->pf, (float)k, n, c->st));
     TRY(matvec32_pre(c, c->Apf, c->rf, 0, false));
-    CK(cudaMemsetAsync(c->xf, 0, n * sizeof(float), c->st));
-    CK(dev_scale_f(c->pf, (float)k, n, c->st));
     CK(dev_dot_k0(c->rf, c->rf, c->N3, c->pre_dev + 36, c->part, c->sc, SC_RRNEW, OP_STORE, c->st));
-    double rr_new;
-    TRY(read_scalar(c, SC_RRNEW, &rr_new));
     // beta = |r_true|^2 / |r_prev|^2 with both in the new scaling (the iteration's beta
     // with the recomputed residual in place of the recursive one)
-    beta = rr_new / (rr_prev * k * k);
-    rr = rr_new;
+    rrk2 = rr_prev * k * k;
     scale = nscale;
   }
   *iters = it;
@@ -1447,10 +1445,11 @@ int tangent_solve_f32(Ctx* c, int i, double tol, int* its) {
     return CPFFT_ERR_NONFINITE;
   }
   if (rn > tol * nb && rr > 0.0) {
-    double rr_out, rr_prev;
-    int it = 0, stop = 0;
-    TRY(cg_segment(c, rr, rn, tol * nb, 0.0, 0.0, 0, 2000, 0.0, &rr_out, &rr_prev, &it, &stop));
-    if (stop == STOP_NONFINITE) { cpfft_set_error("FP32 CG residual is not finite"); return CPFFT_ERR_NONFINITE; }
+    double rr_prev;
+    int it = 0, stop = 0, done = 0;
+    TRY(cg_segment(c, rn, tol * nb, 0.0, 0.0, 0, 2000, 0.0, &done));
+    TRY(read_scalars(c));
+    TRY(cg_segment_end(c, done, &it, &rr_prev, &stop));
     if (stop == STOP_MAXIT) { cpfft_set_error("tangent_homo: FP32 CG did not converge"); return CPFFT_ERR_CG_MAXIT; }
     *its = it;
     c->cg_iters += it;
@@ -1469,9 +1468,8 @@ int tangent_solve_f32(Ctx* c, int i, double tol, int* its) {
 // Column i of C_homo from io = E_i + x: C_homo(j, i) = mean of K : (E_i + x) over the
 // grid, component j (src/tangent_homo.f:60-68); the nine sums read back at once.
 int homo_column(Ctx* c, int i, double* C_homo) {
-  const long long N3 = c->N3, n = 9 * N3;
-  for (int j = 0; j < 9; j++)
-    CK(dev_dot(c->K4 + 9 * j * N3, c->io, n, c->part, c->sc, SC_SUM9 + j, OP_STORE, c->st));
+  const long long N3 = c->N3;
+  CK(dev_homo9(c->K4, c->io, N3, c->part, c->sc, SC_SUM9, c->st));
   CK(cudaMemcpyAsync(c->h_sc + SC_SUM9, c->sc + SC_SUM9, 9 * sizeof(double),
                      cudaMemcpyDeviceToHost, c->st));
   TRY(sync(c));
@@ -1797,7 +1795,7 @@ int cpfft_init(int N, const int* matList, const double* kocks_deg, const cpfft_c
       (tabs.size() && (rc = dalloc(c->ptabs, tabs.size() * sizeof(PowTab)))) ||
       (rc = dalloc(c->S, (size_t)9 * N * N * c->g.H * sizeof(double2))) ||
       (rc = dalloc(c->tw, N * sizeof(double2))) || (rc = dalloc(c->part, (size_t)std::max<long long>(9 * NPART, (long long)N * N) * sizeof(double))) ||
-      (rc = dalloc(c->sc, SC_COUNT * sizeof(double))) || (rc = dalloc(c->bar, sizeof(unsigned))) ||
+      (rc = dalloc(c->sc, SC_ALLOC * sizeof(double))) || (rc = dalloc(c->bar, sizeof(unsigned))) ||
       (rc = dalloc(c->stats, 8 * sizeof(unsigned long long))))
     return fail(rc);
   if (cudaMallocHost((void**)&c->h_sc, SC_COUNT * sizeof(double)) != cudaSuccess ||
@@ -1838,7 +1836,7 @@ int cpfft_init(int N, const int* matList, const double* kocks_deg, const cpfft_c
   if ((e = cudaMemcpy(c->tw, tw.data(), N * sizeof(double2), cudaMemcpyHostToDevice)) ||
       (e = cudaMemcpy(c->Fn, F.data(), f9, cudaMemcpyHostToDevice)) ||
       (e = cudaMemcpy(c->Fn1, F.data(), f9, cudaMemcpyHostToDevice)) ||
-      (e = cudaMemset(c->P, 0, f9)) || (e = cudaMemset(c->K4, 0, 81 * N3 * sizeof(double))) ||
+      (e = cudaMemset(c->sc, 0, SC_ALLOC * sizeof(double))) || (e = cudaMemset(c->P, 0, f9)) || (e = cudaMemset(c->K4, 0, 81 * N3 * sizeof(double))) ||
       (e = cudaMemcpy(c->hist[0], h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice)) ||
       (e = cudaMemcpy(c->hist[1], h.data(), h.size() * sizeof(double), cudaMemcpyHostToDevice)) ||
       (e = cudaMemcpy(c->ori, ori.data(), N3 * sizeof(int), cudaMemcpyHostToDevice)) ||

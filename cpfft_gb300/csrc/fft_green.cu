@@ -75,7 +75,7 @@ template <typename T, bool SPLIT>
 __global__ void __launch_bounds__(256) small_forward(const T* __restrict__ x, const T* __restrict__ K4,
                                                      int flgK, typename Vec2<T>::t* __restrict__ S,
                                                      GridDesc g, const typename Vec2<T>::t* __restrict__ twg,
-                                                     double* __restrict__ part) {
+                                                     double* __restrict__ part, double* scf) {
   using T2 = typename Vec2<T>::t;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int N = g.N;
@@ -99,7 +99,8 @@ __global__ void __launch_bounds__(256) small_forward(const T* __restrict__ x, co
         return s;
       },
       S, i, c0, g, tw, b0, b0 + std::max(plane_cols(N), 3 * SMALL_TKC) * padlen(N));
-  if (part) block_partial<256>((double)dsum, part + blockIdx.x);
+  if (part && scf) grid_sum((double)dsum, part, FinalOp{scf, SC_PAP, OP_ALPHA, 0, 0});
+  else if (part) block_partial<256>((double)dsum, part + blockIdx.x);
 }
 
 template <bool SPLIT>
@@ -140,11 +141,12 @@ constexpr int small_max() { return sizeof(T) == 8 ? 48 : 80; }
 
 template <typename T, bool SPLIT>
 void small_apply(const T* x, const T* K4, int flgK, T* y, typename Vec2<T>::t* S,
-                 const typename Vec2<T>::t* tw, const GridDesc& g, cudaStream_t st, double* part) {
+                 const typename Vec2<T>::t* tw, const GridDesc& g, cudaStream_t st, double* part,
+                 double* scf) {
   const int N = g.N;
   const size_t sm = smem_small<T>(N);
   constexpr int BT = 256;
-  small_forward<T, SPLIT><<<9 * N, BT, sm, st>>>(x, K4, flgK, S, g, tw, part);
+  small_forward<T, SPLIT><<<9 * N, BT, sm, st>>>(x, K4, flgK, S, g, tw, part, scf);
   if constexpr (sizeof(T) == 8) {
     small_columns<SPLIT><<<dim3((g.H + SMALL_TKC - 1) / SMALL_TKC, N, 3), 128, sm, st>>>(S, g, tw);
   } else {
@@ -213,16 +215,16 @@ cudaError_t green_apply_dot(const T* x, const T* K4, int flgK, T* y, typename Ve
   if (rfuse && !warp_path) return cudaErrorNotSupported;  // the fused update needs the warp passes
   if (N <= small_max<T>() && !warp_path) {
     double* part_a = (g.pre && part && flgK) ? part : nullptr;
-    if (part_a && nparts) *nparts = 9 * N;
+    if (part_a && nparts) *nparts = scf ? -1 : 9 * N;
     if constexpr (sizeof(T) == 8) {
       if (N <= 16) {  // split stages: 15^3 33 against 38 us, 20^3 63 against 42
         g.plan = split_plan(N);
-        small_apply<T, true>(x, K4, flgK, y, S, tw, g, st, part_a);
+        small_apply<T, true>(x, K4, flgK, y, S, tw, g, st, part_a, scf);
       } else {
-        small_apply<T, false>(x, K4, flgK, y, S, tw, g, st, part_a);
+        small_apply<T, false>(x, K4, flgK, y, S, tw, g, st, part_a, scf);
       }
     } else {
-      small_apply<T, false>(x, K4, flgK, y, S, tw, g, st, part_a);
+      small_apply<T, false>(x, K4, flgK, y, S, tw, g, st, part_a, scf);
     }
     g_kernel_launches += 3;
     return cudaGetLastError();
@@ -259,12 +261,13 @@ cudaError_t green_apply(const T* x, const T* K4, int flgK, T* y, typename Vec2<T
 
 cudaError_t green_cg_iteration(float* x, float* r, float* p, const float* K4, float2* S,
                                const float2* tw, const GridDesc& g, cudaStream_t st,
-                               double* part_a, double* part_e, const float* k0, double* sc) {
+                               double* part_a, double* part_e, const float* k0, double* sc,
+                               cudaGraphConditionalHandle h, bool uh) {
   switch (g.N) {
-    case 32: wcg_iteration<1>(x, r, p, K4, S, tw, g, st, part_a, part_e, k0, sc); break;
-    case 64: wcg_iteration<2>(x, r, p, K4, S, tw, g, st, part_a, part_e, k0, sc); break;
-    case 128: wcg_iteration<4>(x, r, p, K4, S, tw, g, st, part_a, part_e, k0, sc); break;
-    case 256: wcg_iteration<8>(x, r, p, K4, S, tw, g, st, part_a, part_e, k0, sc); break;
+    case 32: wcg_iteration<1>(x, r, p, K4, S, tw, g, st, part_a, part_e, k0, sc, h, uh); break;
+    case 64: wcg_iteration<2>(x, r, p, K4, S, tw, g, st, part_a, part_e, k0, sc, h, uh); break;
+    case 128: wcg_iteration<4>(x, r, p, K4, S, tw, g, st, part_a, part_e, k0, sc, h, uh); break;
+    case 256: wcg_iteration<8>(x, r, p, K4, S, tw, g, st, part_a, part_e, k0, sc, h, uh); break;
     default: return cudaErrorNotSupported;
   }
   g_kernel_launches += 5;  // the transform passes (dev_final counts its own launch)

@@ -45,7 +45,8 @@ cudaError_t green_apply(const T* x, const T* K4, int flgK, T* y, typename Vec2<T
                         const typename Vec2<T>::t* tw, GridDesc g, cudaStream_t st);
 // the same, and with part != nullptr also the partial sums of x . y: *nparts partials
 // in part (the warp-FFT sizes), or *nparts = 0 when this size does not fuse the product
-// (the caller then reduces x . y itself).  rfuse != nullptr (FP32 warp-FFT sizes only,
+// (the caller then reduces x . y itself); with scf as well, the three-pass grids finish the
+// sum of the reference-medium product (scf[SC_PAP] and alpha) and set *nparts = -1.  rfuse != nullptr (FP32 warp-FFT sizes only,
 // else cudaErrorNotSupported): x is the CG direction p, first updated in place to
 // r + beta p (r = rfuse, beta = scf[SC_BETA]; scf[SC_RR] takes scf[SC_RRNEW])
 template <typename T>
@@ -71,11 +72,12 @@ cudaError_t green_setup(int N);
 // operator, from about a fifth of its time.
 // One preconditioned FP32 CG iteration on the register-FFT grids (32..256), g.pre set:
 // p = r + beta p, y = G0(K : p) with alpha = rr / <K : p, p>, x += alpha p,
-// r -= alpha y, part_e = the (N/2) N block partials of <r, r>_K0 (k0: the 9 x 9 weights);
-// y never reaches memory.  The caller finishes rr_new / beta and the stop test.
+// r -= alpha y, <r, r>_K0 (k0: the 9 x 9 weights; part_a, part_e: (N/2) N partials), beta and
+// the segment's stop test; y never reaches memory.
 cudaError_t green_cg_iteration(float* x, float* r, float* p, const float* K4, float2* S,
                                const float2* tw, const GridDesc& g, cudaStream_t st,
-                               double* part_a, double* part_e, const float* k0, double* sc);
+                               double* part_a, double* part_e, const float* k0, double* sc,
+                               cudaGraphConditionalHandle h, bool use_handle);
 
 bool green_df_supported(int N);
 cudaError_t green_setup_df(int N);

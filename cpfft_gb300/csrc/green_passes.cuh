@@ -6,6 +6,7 @@
 #include "fft_green.cuh"
 #include "fft_warp.cuh"
 #include "krylov.cuh"
+#include "reduce.cuh"
 
 namespace {
 
@@ -1397,16 +1398,18 @@ void wgreen_apply(const TIO* x, const TK* K4, const float* K4lo, int flgK, TIO* 
 
 // One preconditioned FP32 CG iteration's operator and vector work on the register-FFT
 // grids: pass A with p = r + beta p fused (and the partials of <K : p, p>), alpha from
-// them, passes B-D, pass E fused with x += alpha p, r -= alpha G0(K : p) and the partials
-// of <r, r>_K0 (part_e, (N/2) N of them).  g.pre must be set.
+// them, passes B-D, pass E fused with x += alpha p, r -= alpha G0(K : p) and <r, r>_K0, then
+// beta and the segment's stop test.  g.pre must be set.
 template <int M>
 void wcg_iteration(float* x, float* r, float* p, const float* K4, float2* S, const float2* tw,
                    const GridDesc& g, cudaStream_t st, double* part_a, double* part_e,
-                   const float* k0, double* sc) {
+                   const float* k0, double* sc, cudaGraphConditionalHandle h, bool use_handle) {
   constexpr int N = 32 * M;
   constexpr int NA = ncols9<N>();
   wpass_a<M, float, float, float, true><<<(N / 2) * N, 288, smem_w<float>(N, NA), st>>>(
       p, K4, nullptr, 1, S, g, tw, part_a, r, sc, p);
+  // (finishing the sums in the passes' last blocks, as the smaller grids do, costs what it
+  // saves here: 32^3 38 us an iteration either way, 64^3 117 against 127)
   dev_final(part_a, (N / 2) * N, sc, SC_PAP, OP_ALPHA, st);
   wlaunch_b_any<M, float>(g.wtb, S, g, tw, 0, st);
   if (g.wc2 == 4) wlaunch_c2<M, float, 4>(S, g, tw, st);
@@ -1415,6 +1418,7 @@ void wcg_iteration(float* x, float* r, float* p, const float* K4, float2* S, con
   else wlaunch_c<M, float, 2>(S, g, tw, st);
   wlaunch_b_any<M, float>(g.wtb, S, g, tw, 1, st);
   wpass_e_xr<M><<<(N / 2) * N, 288, smem_w<float>(N, NA), st>>>(S, g, tw, x, r, p, k0, sc, part_e);
+  dev_final(part_e, (N / 2) * N, sc, SC_RRNEW, OP_BETA_COND, st, h, use_handle);
 }
 
 template <typename T>

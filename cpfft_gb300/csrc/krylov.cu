@@ -1,55 +1,31 @@
 // krylov.cu -- vector kernels of the device-resident Newton-Krylov loop: CG updates,
-// deterministic two-stage reductions (warp shuffles inside a block, one partial per
-// block, a single-block final pass), field fills and precision casts.
+// deterministic reductions (warp shuffles inside a block, one partial per block, added in a
+// fixed order by the last block, reduce.cuh), field fills and precision casts.
+#include <algorithm>
+
 #include "krylov.cuh"
+#include "reduce.cuh"
 
 namespace {
 
 constexpr int RB = 256;  // threads per reduction block
 
-__device__ __forceinline__ double warp_sum(double v) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
-}
-__device__ __forceinline__ double block_sum(double v) {
-  __shared__ double ws[RB / 32];
-  v = warp_sum(v);
-  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (lane == 0) ws[w] = v;
-  __syncthreads();
-  v = threadIdx.x < RB / 32 ? ws[threadIdx.x] : 0.0;
-  if (w == 0) v = warp_sum(v);
-  return v;  // valid in thread 0
-}
-
 template <typename TA, typename TB>
 __global__ void __launch_bounds__(RB) k_dot(const TA* __restrict__ a, const TB* __restrict__ b,
-                                            long long n, double* __restrict__ part) {
+                                            long long n, double* __restrict__ part, FinalOp f) {
   TA s = 0;
   for (long long i = (long long)blockIdx.x * RB + threadIdx.x; i < n; i += (long long)gridDim.x * RB)
     s += a[i] * (TA)b[i];
-  double sb = block_sum((double)s);
-  if (threadIdx.x == 0) part[blockIdx.x] = sb;
+  grid_sum((double)s, part, f);
 }
 
-// final pass: sc[slot] = sum(part); op-specific scalar follow-ups for CG
-__global__ void __launch_bounds__(1024) k_final(const double* __restrict__ part, int np,
-                                                double* __restrict__ sc, int slot, int op) {
+// sum of partials a transform pass left (grids whose passes do not finish them themselves)
+__global__ void __launch_bounds__(1024) k_final(const double* __restrict__ part, int np, FinalOp f) {
   __shared__ double ws[32];
   double v = 0.0;
   for (int i = threadIdx.x; i < np; i += 1024) v += part[i];
-  v = warp_sum(v);
-  if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    v = ws[threadIdx.x];
-    v = warp_sum(v);
-    if (threadIdx.x == 0) {
-      sc[slot] = v;
-      if (op == OP_ALPHA) sc[SC_ALPHA] = sc[SC_RR] / v;          // alpha = rr / pAp
-      else if (op == OP_BETA) sc[SC_BETA] = v / sc[SC_RR];       // beta = rr_new / rr
-    }
-  }
+  v = block_sum(v, ws);
+  if (threadIdx.x == 0) apply_final(f, v);
 }
 
 // x += alpha p ; r -= alpha Ap ; partial r.r
@@ -57,7 +33,7 @@ template <typename T>
 __global__ void __launch_bounds__(RB) k_cg_xr(T* __restrict__ x, T* __restrict__ r,
                                               const T* __restrict__ p, const T* __restrict__ Ap,
                                               long long n, const double* __restrict__ sc,
-                                              double* __restrict__ part) {
+                                              double* __restrict__ part, FinalOp f) {
   // arithmetic in T: on GB300 an FP64 instruction costs ~64 FP32 ones, so the FP32
   // vectors stay in FP32; per-thread partial sums are promoted only for the block sum
   const T alpha = (T)sc[SC_ALPHA];
@@ -68,8 +44,7 @@ __global__ void __launch_bounds__(RB) k_cg_xr(T* __restrict__ x, T* __restrict__
     r[i] = ri;
     s += ri * ri;
   }
-  double sb = block_sum((double)s);
-  if (threadIdx.x == 0) part[blockIdx.x] = sb;
+  grid_sum((double)s, part, f);
 }
 
 // FP32 form with 16-byte vector accesses (n % 4 elements handled by a scalar tail)
@@ -77,7 +52,7 @@ __global__ void __launch_bounds__(RB) k_cg_xr4(float* __restrict__ x, float* __r
                                                const float* __restrict__ p,
                                                const float* __restrict__ Ap, long long n,
                                                const double* __restrict__ sc,
-                                               double* __restrict__ part) {
+                                               double* __restrict__ part, FinalOp f) {
   const float alpha = (float)sc[SC_ALPHA];
   const long long n4 = n >> 2, stride = (long long)gridDim.x * RB;
   float4* x4 = reinterpret_cast<float4*>(x);
@@ -100,8 +75,7 @@ __global__ void __launch_bounds__(RB) k_cg_xr4(float* __restrict__ x, float* __r
     r[i] = ri;
     s += ri * ri;
   }
-  double sb = block_sum((double)s);
-  if (threadIdx.x == 0) part[blockIdx.x] = sb;
+  grid_sum((double)s, part, f);
 }
 
 __global__ void k_cg_p4(float* __restrict__ p, const float* __restrict__ r, long long n,
@@ -169,6 +143,49 @@ __global__ void k_add_const(double* __restrict__ y, double v, long long n) {
        i += (long long)gridDim.x * blockDim.x)
     y[i] += v;
 }
+// y = s * (double)x_f, x_f = 0
+__global__ void k_take_f32(double* __restrict__ y, float* __restrict__ x, double s, long long n) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    y[i] = s * (double)x[i];
+    x[i] = 0.0f;
+  }
+}
+// y_f = (float)(x * s), p_f *= k
+__global__ void k_restart_f32(float* __restrict__ y, const double* __restrict__ x, double s,
+                              float* __restrict__ p, float k, long long n) {
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
+       i += (long long)gridDim.x * blockDim.x) {
+    y[i] = (float)(x[i] * s);
+    p[i] *= k;
+  }
+}
+// y = a - b and the sum of y^2
+__global__ void __launch_bounds__(RB) k_sub_norm(double* __restrict__ y, const double* __restrict__ a,
+                                                 const double* __restrict__ b, long long n,
+                                                 double* __restrict__ part, FinalOp f) {
+  double s = 0.0;
+  for (long long i = (long long)blockIdx.x * RB + threadIdx.x; i < n; i += (long long)gridDim.x * RB) {
+    const double d = a[i] - b[i];
+    y[i] = d;
+    s += d * d;
+  }
+  grid_sum(s, part, f);
+}
+// the scalars of a CG segment that starts from the <r, r>_K0 in SC_RRNEW
+__global__ void k_cg_start(double* __restrict__ sc, double rn, double tolb, double tol, double delta,
+                           double it, double maxit, double rrk2) {
+  const double rr = sc[SC_RRNEW];
+  sc[SC_BETA] = rrk2 > 0.0 ? rr / rrk2 : 0.0;
+  sc[SC_RR0] = rr;
+  sc[SC_RN] = rn;
+  sc[SC_TOLB] = tolb;
+  sc[SC_TOL] = tol;
+  sc[SC_DELTA] = delta;
+  sc[SC_CNT] = it;
+  sc[SC_MAXIT] = maxit;
+  sc[SC_STOP] = 0.0;
+}
 // y_f = (float)(x * s)
 __global__ void k_to_f32(float* __restrict__ y, const double* __restrict__ x, double s, long long n) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
@@ -181,17 +198,32 @@ __global__ void k_add_f32(double* __restrict__ y, const float* __restrict__ x, d
        i += (long long)gridDim.x * blockDim.x)
     y[i] += s * (double)x[i];
 }
-// sums of each of the 9 components of a (9, N3) field (one partial per block and comp)
+// sums of each of the 9 components of a (9, N3) field
 __global__ void __launch_bounds__(RB) k_sum9(const double* __restrict__ x, long long N3,
-                                             double* __restrict__ part) {
-  for (int c = 0; c < 9; c++) {
-    double s = 0.0;
-    for (long long i = (long long)blockIdx.x * RB + threadIdx.x; i < N3; i += (long long)gridDim.x * RB)
-      s += x[c * N3 + i];
-    s = block_sum(s);
-    if (threadIdx.x == 0) part[c * gridDim.x + blockIdx.x] = s;
-    __syncthreads();
+                                             double* __restrict__ part, double* __restrict__ sc,
+                                             int slot) {
+  double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (long long i = (long long)blockIdx.x * RB + threadIdx.x; i < N3; i += (long long)gridDim.x * RB)
+#pragma unroll
+    for (int c = 0; c < 9; c++) s[c] += x[c * N3 + i];
+  grid_sum9(s, part, sc, slot);
+}
+
+// the nine components of K4 : x summed over the grid (x read once for all nine)
+__global__ void __launch_bounds__(RB) k_homo9(const double* __restrict__ K4, const double* __restrict__ x,
+                                              long long N3, double* __restrict__ part,
+                                              double* __restrict__ sc, int slot) {
+  double s[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (long long v = (long long)blockIdx.x * RB + threadIdx.x; v < N3; v += (long long)gridDim.x * RB) {
+    double xv[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) xv[k] = x[k * N3 + v];
+#pragma unroll
+    for (int j = 0; j < 9; j++)
+#pragma unroll
+      for (int k = 0; k < 9; k++) s[j] += K4[(9 * j + k) * N3 + v] * xv[k];
   }
+  grid_sum9(s, part, sc, slot);
 }
 
 // ---- K0-weighted forms of the reference-medium preconditioned FP32 CG ----------------
@@ -214,14 +246,14 @@ __device__ __forceinline__ float k0_form(const float* s_k0, const float* a, cons
   return s;
 }
 
-// x += alpha p ; r -= alpha Ap ; partial <r, r>_K0 -- one voxel's 9 components per thread
+// x += alpha p ; r -= alpha Ap ; <r, r>_K0 -- one voxel's 9 components per thread
 // (component-major fields), four voxels at a time with 16-byte accesses when N3 % 4 == 0
 __global__ void __launch_bounds__(RB) k_cg_xr_k0(float* __restrict__ x, float* __restrict__ r,
                                                  const float* __restrict__ p,
                                                  const float* __restrict__ Ap, long long N3,
                                                  const float* __restrict__ k0,
                                                  const double* __restrict__ sc,
-                                                 double* __restrict__ part) {
+                                                 double* __restrict__ part, FinalOp f) {
   __shared__ float s_k0[81];
   load_k0(k0, s_k0);
   const float alpha = (float)sc[SC_ALPHA];
@@ -260,14 +292,13 @@ __global__ void __launch_bounds__(RB) k_cg_xr_k0(float* __restrict__ x, float* _
       s += k0_form(s_k0, rv, rv);
     }
   }
-  double sb = block_sum((double)s);
-  if (threadIdx.x == 0) part[blockIdx.x] = sb;
+  grid_sum((double)s, part, f);
 }
 
 // partial <a, b>_K0
 __global__ void __launch_bounds__(RB) k_dot_k0(const float* __restrict__ a, const float* __restrict__ b,
                                                long long N3, const float* __restrict__ k0,
-                                               double* __restrict__ part) {
+                                               double* __restrict__ part, FinalOp f) {
   __shared__ float s_k0[81];
   load_k0(k0, s_k0);
   float s = 0.f;
@@ -277,8 +308,7 @@ __global__ void __launch_bounds__(RB) k_dot_k0(const float* __restrict__ a, cons
     for (int i = 0; i < 9; i++) { av[i] = a[i * N3 + v]; bv[i] = b[i * N3 + v]; }
     s += k0_form(s_k0, av, bv);
   }
-  double sb = block_sum((double)s);
-  if (threadIdx.x == 0) part[blockIdx.x] = sb;
+  grid_sum((double)s, part, f);
 }
 
 // component sums of an (81, N3) FP32 field: part[m * gridDim.x + blockIdx.x]
@@ -288,7 +318,8 @@ __global__ void __launch_bounds__(RB) k_sum81(const float* __restrict__ K, long 
   double s = 0.0;
   for (long long v = (long long)blockIdx.x * RB + threadIdx.x; v < N3; v += (long long)gridDim.x * RB)
     s += (double)K[m * N3 + v];
-  s = block_sum(s);
+  __shared__ double ws[32];
+  s = block_sum(s, ws);
   if (threadIdx.x == 0) part[m * gridDim.x + blockIdx.x] = s;
 }
 
@@ -301,24 +332,6 @@ __global__ void __launch_bounds__(64) k_final_rows(const double* __restrict__ pa
   if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
   __syncthreads();
   if (threadIdx.x == 0) out[blockIdx.x] = ws[0] + ws[1];
-}
-
-__global__ void k_cg_cond(double* __restrict__ sc, cudaGraphConditionalHandle h, int use_handle) {
-  const double rr = sc[SC_RRNEW];
-  const double cnt = sc[SC_CNT] + 1.0;
-  sc[SC_CNT] = cnt;
-  int stop = STOP_NONE;
-  if (!isfinite(rr)) {
-    stop = STOP_NONFINITE;
-  } else if (!(sc[SC_RR0] > 0.0)) {
-    stop = STOP_TEST;  // nothing to reduce: let the caller's true residual decide
-  } else {
-    const double red = sqrt(fmax(rr, 0.0) / sc[SC_RR0]), est = sc[SC_RN] * red;
-    if (red < sc[SC_DELTA] || est <= sc[SC_TOLB] || est <= sc[SC_TOL]) stop = STOP_TEST;
-    else if (cnt >= sc[SC_MAXIT]) stop = STOP_MAXIT;
-  }
-  sc[SC_STOP] = (double)stop;
-  if (use_handle) cudaGraphSetConditional(h, stop == STOP_NONE ? 1u : 0u);
 }
 
 // The iteration graph's first node: its WHILE loop runs only if the iterations are not
@@ -340,28 +353,29 @@ static cudaError_t counted(int k) {
   return cudaGetLastError();
 }
 
+// blocks of a reduction over n values: enough for every SM, at most NPART
+static int blocks_for(long long n) { return (int)std::max<long long>(1, std::min<long long>(NPART, (n + RB - 1) / RB)); }
+
 cudaError_t dev_dot(const double* a, const double* b, long long n, double* part, double* sc,
                     int slot, int op, cudaStream_t st) {
-  k_dot<double, double><<<NPART, RB, 0, st>>>(a, b, n, part);
-  k_final<<<1, 1024, 0, st>>>(part, NPART, sc, slot, op);
-  return counted(2);
+  k_dot<double, double><<<blocks_for(n), RB, 0, st>>>(a, b, n, part, FinalOp{sc, slot, op, 0, 0});
+  return counted(1);
 }
 cudaError_t dev_dot_f(const float* a, const float* b, long long n, double* part, double* sc,
                       int slot, int op, cudaStream_t st) {
-  k_dot<float, float><<<NPART, RB, 0, st>>>(a, b, n, part);
-  k_final<<<1, 1024, 0, st>>>(part, NPART, sc, slot, op);
-  return counted(2);
+  k_dot<float, float><<<blocks_for(n), RB, 0, st>>>(a, b, n, part, FinalOp{sc, slot, op, 0, 0});
+  return counted(1);
 }
 template <typename T>
 cudaError_t dev_cg_xr(T* x, T* r, const T* p, const T* Ap, long long n, double* part, double* sc,
                       cudaStream_t st) {
+  const FinalOp f{sc, SC_RRNEW, OP_BETA, 0, 0};
   if (sizeof(T) == 4)
-    k_cg_xr4<<<NPART, RB, 0, st>>>((float*)x, (float*)r, (const float*)p, (const float*)Ap, n,
-                                   sc, part);
+    k_cg_xr4<<<blocks_for(n / 4), RB, 0, st>>>((float*)x, (float*)r, (const float*)p, (const float*)Ap,
+                                               n, sc, part, f);
   else
-    k_cg_xr<T><<<NPART, RB, 0, st>>>(x, r, p, Ap, n, sc, part);
-  k_final<<<1, 1024, 0, st>>>(part, NPART, sc, SC_RRNEW, OP_BETA);
-  return counted(2);
+    k_cg_xr<T><<<blocks_for(n), RB, 0, st>>>(x, r, p, Ap, n, sc, part, f);
+  return counted(1);
 }
 template <typename T>
 cudaError_t dev_cg_p(T* p, const T* r, long long n, double* sc, cudaStream_t st) {
@@ -371,8 +385,9 @@ cudaError_t dev_cg_p(T* p, const T* r, long long n, double* sc, cudaStream_t st)
     k_cg_p<T><<<grid_for(n, 256), 256, 0, st>>>(p, r, n, sc);
   return counted(1);
 }
-cudaError_t dev_final(double* part, int np, double* sc, int slot, int op, cudaStream_t st) {
-  k_final<<<1, 1024, 0, st>>>(part, np, sc, slot, op);
+cudaError_t dev_final(double* part, int np, double* sc, int slot, int op, cudaStream_t st,
+                      cudaGraphConditionalHandle h, bool use_handle) {
+  k_final<<<1, 1024, 0, st>>>(part, np, FinalOp{sc, slot, op, h, use_handle ? 1 : 0});
   return counted(1);
 }
 template cudaError_t dev_cg_xr<double>(double*, double*, const double*, const double*, long long,
@@ -415,25 +430,47 @@ cudaError_t dev_add_f32(double* y, const float* x, double s, long long n, cudaSt
   k_add_f32<<<grid_for(n, 256), 256, 0, st>>>(y, x, s, n);
   return counted(1);
 }
+cudaError_t dev_take_f32(double* y, float* x, double s, long long n, cudaStream_t st) {
+  k_take_f32<<<grid_for(n, 256), 256, 0, st>>>(y, x, s, n);
+  return counted(1);
+}
+cudaError_t dev_restart_f32(float* y, const double* x, double s, float* p, float k, long long n,
+                            cudaStream_t st) {
+  k_restart_f32<<<grid_for(n, 256), 256, 0, st>>>(y, x, s, p, k, n);
+  return counted(1);
+}
+cudaError_t dev_sub_norm(double* y, const double* a, const double* b, long long n, double* part,
+                         double* sc, int slot, cudaStream_t st) {
+  k_sub_norm<<<blocks_for(n), RB, 0, st>>>(y, a, b, n, part, FinalOp{sc, slot, OP_STORE, 0, 0});
+  return counted(1);
+}
+cudaError_t dev_cg_start(double* sc, double rn, double tolb, double tol, double delta, int it,
+                         int maxit, double rrk2, cudaStream_t st) {
+  k_cg_start<<<1, 1, 0, st>>>(sc, rn, tolb, tol, delta, (double)it, (double)maxit, rrk2);
+  return counted(1);
+}
 cudaError_t dev_sum9(const double* x, long long N3, double* part, double* sc, int slot0,
                      cudaStream_t st) {
-  k_sum9<<<NPART, RB, 0, st>>>(x, N3, part);
-  for (int c = 0; c < 9; c++)
-    k_final<<<1, 1024, 0, st>>>(part + c * NPART, NPART, sc, slot0 + c, OP_STORE);
-  return counted(10);
+  k_sum9<<<blocks_for(N3), RB, 0, st>>>(x, N3, part, sc, slot0);
+  return counted(1);
+}
+cudaError_t dev_homo9(const double* K4, const double* x, long long N3, double* part, double* sc,
+                      int slot, cudaStream_t st) {
+  k_homo9<<<blocks_for(N3), RB, 0, st>>>(K4, x, N3, part, sc, slot);
+  return counted(1);
 }
 
 cudaError_t dev_cg_xr_k0(float* x, float* r, const float* p, const float* Ap, long long N3,
-                         const float* k0, double* part, double* sc, cudaStream_t st) {
-  k_cg_xr_k0<<<NPART, RB, 0, st>>>(x, r, p, Ap, N3, k0, sc, part);
-  k_final<<<1, 1024, 0, st>>>(part, NPART, sc, SC_RRNEW, OP_BETA);
-  return counted(2);
+                         const float* k0, double* part, double* sc, cudaGraphConditionalHandle h,
+                         bool use_handle, cudaStream_t st) {
+  k_cg_xr_k0<<<blocks_for(N3), RB, 0, st>>>(x, r, p, Ap, N3, k0, sc, part,
+                                            FinalOp{sc, SC_RRNEW, OP_BETA_COND, h, use_handle ? 1 : 0});
+  return counted(1);
 }
 cudaError_t dev_dot_k0(const float* a, const float* b, long long N3, const float* k0,
                        double* part, double* sc, int slot, int op, cudaStream_t st) {
-  k_dot_k0<<<NPART, RB, 0, st>>>(a, b, N3, k0, part);
-  k_final<<<1, 1024, 0, st>>>(part, NPART, sc, slot, op);
-  return counted(2);
+  k_dot_k0<<<blocks_for(N3), RB, 0, st>>>(a, b, N3, k0, part, FinalOp{sc, slot, op, 0, 0});
+  return counted(1);
 }
 cudaError_t dev_mean81(const float* K, long long N3, double* part, double* sc81, cudaStream_t st) {
   constexpr int NB = 64;
@@ -441,12 +478,6 @@ cudaError_t dev_mean81(const float* K, long long N3, double* part, double* sc81,
   k_final_rows<<<81, 64, 0, st>>>(part, NB, sc81);
   return counted(2);
 }
-cudaError_t dev_cg_cond(double* sc, cudaGraphConditionalHandle h, bool use_handle,
-                        cudaStream_t st) {
-  k_cg_cond<<<1, 1, 0, st>>>(sc, h, use_handle ? 1 : 0);
-  return counted(1);
-}
-
 cudaError_t dev_cg_gate(const double* sc, cudaGraphConditionalHandle h, cudaStream_t st) {
   k_cg_gate<<<1, 1, 0, st>>>(sc, h);
   return counted(1);
