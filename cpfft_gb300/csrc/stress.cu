@@ -12,7 +12,7 @@
 // tangent and the rotation, contractions with the trace-free Schmid tensors take five
 // products, and cep2A's 81-term loops are contracted through 3x3 intermediates (about 1.6
 // kflop instead of ~20 kflop).  One implicit pass with the reference's start on a GB300: 64^3
-// FCC Voce 22.5 to 15.7 ms, 32^3 BCC-48 (exponent 5.48) 12.3 to 4.4 ms.  Every local loop is
+// FCC Voce 22.5 to 14.7 ms, 32^3 BCC-48 (exponent 5.48) 12.4 to 4.3 ms.  Every local loop is
 // bounded by miter and the line-search cap, so no thread can spin.
 #include <algorithm>
 
@@ -222,19 +222,21 @@ __device__ __forceinline__ void symsw(const double* s, const double* w, double* 
   sw[5] = 0.5 * (w[1] * (s[0] - s[2]) + w[0] * s[3] - w[2] * s[4]);
 }
 
-// LU with partial pivoting, in place, n <= 18, one right-hand side.  The pivots'
-// reciprocals are formed once (a division costs about six FP64 instructions).
+// magnitude of a value's high word: orders magnitudes to 2^-20 without an FP64 comparison
+__device__ __forceinline__ int mag(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+// LU with partial pivoting (on the high words), in place, n <= 7, one right-hand side.  The
+// pivots' reciprocals are formed once (a division costs about six FP64 instructions).
 template <int n>
-__device__ bool lu_solve1(double* a, double* b) {
+__device__ void lu_solve1(double* a, double* b) {
   double inv[n];
   for (int k = 0; k < n; k++) {
-    int p = k;
-    double best = fabs(a[k * n + k]);
+    int p = k, best = mag(a[k * n + k]);
     for (int i = k + 1; i < n; i++) {
-      double v = fabs(a[i * n + k]);
+      const int v = mag(a[i * n + k]);
       if (v > best) { best = v; p = i; }
     }
-    if (best == 0.0) return false;
+    if (best == 0) return;
     if (p != k) {
       for (int j = k; j < n; j++) { double t = a[k * n + j]; a[k * n + j] = a[p * n + j]; a[p * n + j] = t; }
       double t = b[k]; b[k] = b[p]; b[p] = t;
@@ -251,7 +253,6 @@ __device__ bool lu_solve1(double* a, double* b) {
     for (int k = i + 1; k < n; k++) s -= a[i * n + k] * b[k];
     b[i] = s * inv[i];
   }
-  return true;
 }
 
 // ---- mm10 Voce crystal (one crystal per voxel) ---------------------------------------
@@ -267,8 +268,9 @@ struct Crystal {
   double ms[NS][6];
   double qc[NS][3];
   double Cms[NS][6];  // C ms_i, constant while ms is (the reference forms it per call)
-  // the last residual's resolved shears, slip increments, |rs|^(n-1) and dg / tt^n
-  double rs[NS], si[NS], pw[NS], dgn;
+  // the last residual's resolved shears, slip increments, |rs|^(n-1), dg / tt^n, sum of slip
+  // increments times qc, and (R2) sum of |si|
+  double rs[NS], si[NS], pw[NS], dgn, w[3], gsum;
   // MTS: shear modulus and thresholds of this (sub)step, the n-state values of the history's
   // u words (nu1, nu2 < 0: first step), and the temperature of the (sub)step
   double mu, tau_y, tau_v, ntau_y, nmu, nu1, nu2, temp;
@@ -380,7 +382,7 @@ __device__ __forceinline__ double hpow(const CrysRec& c, double h) {
 }
 
 // R1 (mm10_formR1, src/mm10_b.f:1061-1101) from the last slips
-__device__ void formR1(const Crystal& s, const double* st, double* R1) {
+__device__ void formR1(Crystal& s, const double* st, double* R1) {
   const CrysRec& c = *s.cr;
   double dbar[6] = {0, 0, 0, 0, 0, 0}, w[3] = {0, 0, 0};
   double tid = s.tinc * c.iD_v;
@@ -393,6 +395,7 @@ __device__ void formR1(const Crystal& s, const double* st, double* R1) {
   }
   dbar[2] = -(dbar[0] + dbar[1]);
   double sw[6], wv[6];
+  for (int a = 0; a < 3; a++) s.w[a] = w[a];
   symsw(st, w, sw);
   for (int a = 0; a < 6; a++) wv[a] = s.D[a] - dbar[a];
   for (int a = 0; a < 6; a++) {
@@ -403,10 +406,11 @@ __device__ void formR1(const Crystal& s, const double* st, double* R1) {
 }
 
 // R2 (mm10_formR2 / mm10_h_voche) from the last slips; returns the tau_tilde rate
-__device__ double formR2(const Crystal& s, double tt, double* R2) {
+__device__ double formR2(Crystal& s, double tt, double* R2) {
   const CrysRec& c = *s.cr;
   double g = 0.0, h;
   for (int i = 0; i < NS; i++) g += fabs(s.si[i]);
+  s.gsum = g;
   if constexpr (MTS) {  // mm10_h_mts (src/mm10_b.f:2080-2108)
     h = pow(mts_base(s, mts_cta(s, tt)), c.voce_m) * g;
     h = c.tau_a * (1.0 - s.mu / s.nmu) + (s.mu / c.mu_0) * (s.tau_y - s.ntau_y) +
@@ -436,7 +440,7 @@ __device__ void formJ11(const Crystal& s, const double* st, double* J, double* J
   // d si / d rs = dg n |rs|^(n-1) / tt^n (mm10_dgdt_voche)
   const double fac = s.dgn * c.rate_n, tid = s.tinc * c.iD_v;
   const double nt = -c.rate_n * itt;  // d si / d tt = -n si / tt (mm10_dgdh_voche)
-  double w[3] = {0, 0, 0};
+  const double* w = s.w;
   // 2 symsw(st, q) with the stress differences formed once
   const double t3 = 2.0 * st[3], t4 = 2.0 * st[4], t5 = 2.0 * st[5];
   const double d01 = st[0] - st[1], d12 = st[1] - st[2], d02 = st[0] - st[2];
@@ -462,10 +466,6 @@ __device__ void formJ11(const Crystal& s, const double* st, double* J, double* J
       const double dgdtt = nt * s.si[i];
       for (int a = 0; a < 6; a++) J12[a] += wv[a] * dgdtt;
     }
-    const double f = s.rs[i] * tid + s.si[i];
-    w[0] += f * q0;
-    w[1] += f * q1;
-    w[2] += f * q2;
   }
   for (int a = 0; a < 6; a++) J[ld * a + 2] = -(J[ld * a] + J[ld * a + 1]);
   // mm10_iw (src/mm10_b.f:1590-1634) and the identity
@@ -485,14 +485,17 @@ __device__ void formJ(const Crystal& s, const double* x, double* J) {
   double J12[6] = {0, 0, 0, 0, 0, 0}, et[6] = {0, 0, 0, 0, 0, 0};
   formJ11<7, true>(s, x, J, J12, itt);
   // sum of |rs|^(n-1) sign(rs) ms (mm10_estress_*), of |si| and of |si| sign(1, si)
-  double g = 0.0, gs = 0.0;
+  const double g = s.gsum;
+  double gs = g;
+  if (!c.exact_j22) {
+    gs = 0.0;
+    for (int i = 0; i < NS; i++) gs += s.si[i];
+  }
   for (int i = 0; i < NS; i++) {
     const double r2 = copysign(s.pw[i], s.rs[i]);
     et[0] += r2 * s.ms[i][0];
     et[1] += r2 * s.ms[i][1];
     for (int a = 3; a < 6; a++) et[a] += r2 * s.ms[i][a];
-    g += fabs(s.si[i]);
-    gs += s.si[i];
   }
   et[2] = -(et[0] + et[1]);
   if (c.n_int < 0 && c.rate_n < 2.0) {  // |rs|^(n-2) rs of the reference: NaN at rs = 0
@@ -512,7 +515,7 @@ __device__ void formJ(const Crystal& s, const double* x, double* J) {
     const double ht = hterm(c, tt), hp = hpow(c, ht), sh = sgn1(ht);
     // mm10_ehard_voche; exact_j22 = 0 keeps the reference's extra sign(1, si)
     const double ta = c.voce_m * (-c.inv_tau_v) / fabs(ht) * g;
-    const double tb = c.rate_n * itt * sh * (c.exact_j22 ? g : gs);
+    const double tb = c.rate_n * itt * sh * gs;
     fac = c.theta_0 * s.dgn * c.rate_n * hp * sh;
     J[48] = 1.0 - c.theta_0 * ((ta - tb) * hp);
   }
@@ -576,7 +579,8 @@ __device__ void mts_tangent_rhs(const Crystal& s, const double* st, double tt, c
 
 __device__ __forceinline__ bool anynan(const double* x, int n) {
   bool r = false;
-  for (int i = 0; i < n; i++) r |= isnan(x[i]);
+  for (int i = 0; i < n; i++)  // NaN by the bits
+    r |= mag(x[i]) > 0x7ff00000 || (mag(x[i]) == 0x7ff00000 && __double2loint(x[i]) != 0);
   return r;
 }
 
@@ -1245,9 +1249,9 @@ __device__ void voxel_update(const StressArgs& a, long long v, bool valid, int& 
       double inv[6];
       for (int k = 0; k < 6; k++) {
         int p = k;
-        double best = fabs(JJ[6 * k + k]);
+        int best = mag(JJ[6 * k + k]);
         for (int i = k + 1; i < 6; i++)
-          if (fabs(JJ[6 * i + k]) > best) { best = fabs(JJ[6 * i + k]); p = i; }
+          if (mag(JJ[6 * i + k]) > best) { best = mag(JJ[6 * i + k]); p = i; }
         piv[k] = p;
         if (p != k)
           for (int j = 0; j < 6; j++) { double t = JJ[6 * k + j]; JJ[6 * k + j] = JJ[6 * p + j]; JJ[6 * p + j] = t; }
