@@ -12,7 +12,7 @@
 // tangent and the rotation, contractions with the trace-free Schmid tensors take five
 // products, and cep2A's 81-term loops are contracted through 3x3 intermediates (about 1.6
 // kflop instead of ~20 kflop).  One implicit pass with the reference's start on a GB300: 64^3
-// FCC Voce 22.5 to 14.7 ms, 32^3 BCC-48 (exponent 5.48) 12.4 to 4.3 ms.  Every local loop is
+// FCC Voce 22.5 to 14.7 ms, 32^3 BCC-48 (exponent 5.48) 12.4 to 3.7 ms.  Every local loop is
 // bounded by miter and the line-search cap, so no thread can spin.
 #include <algorithm>
 
@@ -256,6 +256,11 @@ __device__ void lu_solve1(double* a, double* b) {
 }
 
 // ---- mm10 Voce crystal (one crystal per voxel) ---------------------------------------
+// Form of the Jacobian's sum over the systems (formJ11): by rank-one terms, or through sums that
+// the stiffness and the stress multiply once (16 products fewer a system, 276 more a Jacobian).
+// 32^3 BCC-48 4.27 to 3.73 ms by sums; 64^3 FCC (12 systems) 14.5 by terms, 14.8 by sums.
+constexpr bool SUMMED_J = NS > 17;
+
 struct Crystal {
   const CrysRec* cr;
   const double* C;       // global 6x6 (orientation record)
@@ -267,7 +272,7 @@ struct Crystal {
   double tinc, dg;
   double ms[NS][6];
   double qc[NS][3];
-  double Cms[NS][6];  // C ms_i, constant while ms is (the reference forms it per call)
+  double Cms[SUMMED_J ? 1 : NS][6];  // C ms_i, constant while ms is (per call in the reference)
   // the last residual's resolved shears, slip increments, |rs|^(n-1), dg / tt^n, sum of slip
   // increments times qc, and (R2) sum of |si|
   double rs[NS], si[NS], pw[NS], dgn, w[3], gsum;
@@ -297,7 +302,7 @@ __device__ void setup_np1(Crystal& s, const OriRec* rec, const double* D, double
   rt2rve(tr, RE);
   mm3(R, tr, work);
   rt2rvw(work, RWC);
-  double c0[6], c1[6];
+  [[maybe_unused]] double c0[6], c1[6];
   for (int a = 0; a < 6; a++) {
     c0[a] = Cv(s.C, a, 0) - Cv(s.C, a, 2);
     c1[a] = Cv(s.C, a, 1) - Cv(s.C, a, 2);
@@ -316,8 +321,9 @@ __device__ void setup_np1(Crystal& s, const OriRec* rec, const double* D, double
     // the first three components of ms sum to zero (b . n = 0, kept by the rotation), so every
     // contraction with ms takes five products: sum_j v_j ms_j = (v_0 - v_2) ms_0 + (v_1 - v_2)
     // ms_1 + v_3 ms_3 + v_4 ms_4 + v_5 ms_5
-    for (int a = 0; a < 6; a++)
-      s.Cms[i][a] = c0[a] * s.ms[i][0] + c1[a] * s.ms[i][1] + Cv(s.C, a, 3) * s.ms[i][3] +
+    if constexpr (!SUMMED_J)
+      for (int a = 0; a < 6; a++)
+        s.Cms[i][a] = c0[a] * s.ms[i][0] + c1[a] * s.ms[i][1] + Cv(s.C, a, 3) * s.ms[i][3] +
                     Cv(s.C, a, 4) * s.ms[i][4] + Cv(s.C, a, 5) * s.ms[i][5];
   }
 }
@@ -435,8 +441,6 @@ __device__ double formR(Crystal& s, const double* x, double* R) {
 template <int ld, bool WITH12>
 __device__ void formJ11(const Crystal& s, const double* st, double* J, double* J12, double itt) {
   const CrysRec& c = *s.cr;
-  for (int a = 0; a < 6; a++)
-    for (int b = 0; b < 6; b++) J[ld * a + b] = 0.0;
   // d si / d rs = dg n |rs|^(n-1) / tt^n (mm10_dgdt_voche)
   const double fac = s.dgn * c.rate_n, tid = s.tinc * c.iD_v;
   const double nt = -c.rate_n * itt;  // d si / d tt = -n si / tt (mm10_dgdh_voche)
@@ -444,29 +448,102 @@ __device__ void formJ11(const Crystal& s, const double* st, double* J, double* J
   // 2 symsw(st, q) with the stress differences formed once
   const double t3 = 2.0 * st[3], t4 = 2.0 * st[4], t5 = 2.0 * st[5];
   const double d01 = st[0] - st[1], d12 = st[1] - st[2], d02 = st[0] - st[2];
-  for (int i = 0; i < NS; i++) {
-    const double dgdt = fac * s.pw[i] + tid;
-    const double q0 = s.qc[i][0], q1 = s.qc[i][1], q2 = s.qc[i][2];
-    double wv[6];
-    wv[0] = s.Cms[i][0] + t3 * q2 - t5 * q1;
-    wv[1] = s.Cms[i][1] + t3 * q2 - t4 * q0;
-    wv[2] = s.Cms[i][2] + t5 * q1 + t4 * q0;
-    wv[3] = s.Cms[i][3] + q2 * d01 + q0 * st[5] - q1 * st[4];
-    wv[4] = s.Cms[i][4] + q0 * d12 + q1 * st[3] + q2 * st[5];
-    wv[5] = s.Cms[i][5] + q1 * d02 + q0 * st[3] - q2 * st[4];
-    // column 2 is minus the sum of columns 0 and 1 (ms is trace free): formed after the loop
+  if constexpr (SUMMED_J) {
+    // sum_i (C ms_i + B qc_i) (x) g_i ms_i = C M + B Z with 2 symsw(st, q) = B q, M = sum g_i
+    // ms_i (x) ms_i (symmetric, five components) and Z = sum g_i qc_i (x) ms_i; J12 likewise
+    double M[15], Z[15], m12[5] = {0, 0, 0, 0, 0}, z12[3] = {0, 0, 0};
 #pragma unroll
-    for (int b = 0; b < 6; b++) {
-      if (b == 2) continue;
-      const double t = dgdt * s.ms[i][b];
+    for (int k = 0; k < 15; k++) { M[k] = 0.0; Z[k] = 0.0; }
+    for (int i = 0; i < NS; i++) {
+      const double g = fac * s.pw[i] + tid;
+      const double m[5] = {s.ms[i][0], s.ms[i][1], s.ms[i][3], s.ms[i][4], s.ms[i][5]};
+      double t[5];
 #pragma unroll
-      for (int a = 0; a < 6; a++) J[ld * a + b] += wv[a] * t;
+      for (int k = 0; k < 5; k++) t[k] = g * m[k];
+      int e = 0;
+#pragma unroll
+      for (int k = 0; k < 5; k++)
+#pragma unroll
+        for (int l = k; l < 5; l++) M[e++] += m[k] * t[l];
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        const double qq = s.qc[i][q];
+#pragma unroll
+        for (int k = 0; k < 5; k++) Z[5 * q + k] += qq * t[k];
+        if (WITH12) z12[q] += s.si[i] * qq;
+      }
+      if (WITH12) {
+#pragma unroll
+        for (int k = 0; k < 5; k++) m12[k] += s.si[i] * m[k];
+      }
     }
-    if (WITH12) {  // the same (C ms + 2 symTW) vector drives J12 (mm10_formJ12)
-      const double dgdtt = nt * s.si[i];
-      for (int a = 0; a < 6; a++) J12[a] += wv[a] * dgdtt;
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+      const int col = k < 2 ? k : k + 1;
+      const double z0 = Z[k], z1 = Z[5 + k], z2 = Z[10 + k];
+      J[ld * 0 + col] = t3 * z2 - t5 * z1;
+      J[ld * 1 + col] = t3 * z2 - t4 * z0;
+      J[ld * 2 + col] = t5 * z1 + t4 * z0;
+      J[ld * 3 + col] = z2 * d01 + z0 * st[5] - z1 * st[4];
+      J[ld * 4 + col] = z0 * d12 + z1 * st[3] + z2 * st[5];
+      J[ld * 5 + col] = z1 * d02 + z0 * st[3] - z2 * st[4];
+    }
+    if (WITH12) {
+      J12[0] = t3 * z12[2] - t5 * z12[1];
+      J12[1] = t3 * z12[2] - t4 * z12[0];
+      J12[2] = t5 * z12[1] + t4 * z12[0];
+      J12[3] = z12[2] * d01 + z12[0] * st[5] - z12[1] * st[4];
+      J12[4] = z12[0] * d12 + z12[1] * st[3] + z12[2] * st[5];
+      J12[5] = z12[1] * d02 + z12[0] * st[3] - z12[2] * st[4];
+    }
+    for (int a = 0; a < 6; a++) {
+      const double c2 = Cv(s.C, a, 2);
+      const double c5[5] = {Cv(s.C, a, 0) - c2, Cv(s.C, a, 1) - c2, Cv(s.C, a, 3), Cv(s.C, a, 4),
+                            Cv(s.C, a, 5)};
+#pragma unroll
+      for (int k = 0; k < 5; k++) {
+        double v = J[ld * a + (k < 2 ? k : k + 1)];
+#pragma unroll
+        for (int j = 0; j < 5; j++) {
+          const int lo = j < k ? j : k, hi = j < k ? k : j;
+          v += c5[j] * M[lo * 5 - lo * (lo - 1) / 2 + hi - lo];
+        }
+        J[ld * a + (k < 2 ? k : k + 1)] = v;
+      }
+      if (WITH12) {
+        double v = J12[a];
+#pragma unroll
+        for (int j = 0; j < 5; j++) v += c5[j] * m12[j];
+        J12[a] = nt * v;
+      }
+    }
+  } else {
+    for (int a = 0; a < 6; a++)
+      for (int b = 0; b < 6; b++) J[ld * a + b] = 0.0;
+    for (int i = 0; i < NS; i++) {
+      const double dgdt = fac * s.pw[i] + tid;
+      const double q0 = s.qc[i][0], q1 = s.qc[i][1], q2 = s.qc[i][2];
+      double wv[6];
+      wv[0] = s.Cms[i][0] + t3 * q2 - t5 * q1;
+      wv[1] = s.Cms[i][1] + t3 * q2 - t4 * q0;
+      wv[2] = s.Cms[i][2] + t5 * q1 + t4 * q0;
+      wv[3] = s.Cms[i][3] + q2 * d01 + q0 * st[5] - q1 * st[4];
+      wv[4] = s.Cms[i][4] + q0 * d12 + q1 * st[3] + q2 * st[5];
+      wv[5] = s.Cms[i][5] + q1 * d02 + q0 * st[3] - q2 * st[4];
+#pragma unroll
+      for (int b = 0; b < 6; b++) {
+        if (b == 2) continue;
+        const double t = dgdt * s.ms[i][b];
+#pragma unroll
+        for (int a = 0; a < 6; a++) J[ld * a + b] += wv[a] * t;
+      }
+      if (WITH12) {  // the same (C ms + 2 symTW) vector drives J12 (mm10_formJ12)
+        const double dgdtt = nt * s.si[i];
+        for (int a = 0; a < 6; a++) J12[a] += wv[a] * dgdtt;
+      }
     }
   }
+  // column 2 is minus the sum of columns 0 and 1 (ms is trace free)
   for (int a = 0; a < 6; a++) J[ld * a + 2] = -(J[ld * a] + J[ld * a + 1]);
   // mm10_iw (src/mm10_b.f:1590-1634) and the identity
   J[ld * 0 + 3] += 2.0 * w[2];  J[ld * 0 + 5] -= 2.0 * w[1];
@@ -539,9 +616,10 @@ __device__ void mts_tangent_rhs(const Crystal& s, const double* st, double tt, c
   double sq1[6];
   symsw(st, s.qc[0], sq1);
   // JA: sum_i wv_i (x) (alpha si_i d_mod)
+  static_assert(!MTS || !SUMMED_J, "C ms_i is kept");
   for (int i = 0; i < NS; i++) {
     double wv[6];
-    for (int a = 0; a < 6; a++) wv[a] = s.Cms[i][a] + 2.0 * sq1[a];
+    for (int a = 0; a < 6; a++) wv[a] = s.Cms[SUMMED_J ? 0 : i][a] + 2.0 * sq1[a];
     const double g = alpha * s.si[i];
     for (int a = 0; a < 6; a++)
       for (int b = 0; b < 6; b++) JR[6 * a + b] -= wv[a] * (g * dm[b]);
