@@ -37,6 +37,14 @@ FftPlan make_plan(int N);
 // the padding spreads those strides across the 32 banks.
 __host__ __device__ __forceinline__ int pidx(int k) { return k + (k >> 3); }
 __host__ __device__ __forceinline__ int padlen(int N) { return N + (N >> 3) + 1; }
+// The register-FFT passes index their columns by element size.  8-byte elements move 16 lanes a
+// cycle: k + 2 (k / 16) puts both 16 consecutive elements and the transform's rows of P = 8 or
+// 16 into distinct banks (k + k / 8 folds one of 16 consecutive onto another).  16-byte
+// elements move 8 lanes a cycle and keep k + k / 8.
+template <typename T2>
+__host__ __device__ __forceinline__ int widx(int k) {
+  return sizeof(T2) == 8 ? k + 2 * (k >> 4) : pidx(k);
+}
 
 // y = G(K4 : x) (flgK = 1) or y = G(x); S is the spectral scratch (9 * N * N * H complex),
 // tw the length-N forward twiddle table.  All on stream st.

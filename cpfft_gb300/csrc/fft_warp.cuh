@@ -96,7 +96,7 @@ template <> struct Shape<64> { static constexpr int P = 8, R = 8; };
 template <> struct Shape<128> { static constexpr int P = 16, R = 8; };
 template <> struct Shape<256> { static constexpr int P = 16, R = 16; };
 
-// Transform the column at col (element k at col[pidx(k)]) with thread t of its P threads;
+// Transform the column at col (element k at col[widx(k)]) with thread t of its P threads;
 // tw[k] = exp(-2 pi i k / N) in shared memory.  Every lane of the warp must call this
 // (warp-synchronous shuffles and __syncwarp), each on its own column.
 template <int N, typename T2, typename T, bool INV>
@@ -105,7 +105,7 @@ __device__ __forceinline__ void column(T2* col, const T2* tw, int t) {
   T2 v[R > P ? R : P];
 #pragma unroll
   for (int j = 0; j < R; j++) {
-    v[j] = col[pidx(t + P * j)];
+    v[j] = col[widx<T2>(t + P * j)];
     if (INV) v[j].y = -v[j].y;
   }
   dft<R, T2, T>(v);
@@ -113,23 +113,23 @@ __device__ __forceinline__ void column(T2* col, const T2* tw, int t) {
   for (int k1 = 1; k1 < R; k1++) v[k1] = cmul(v[k1], tw[t * k1]);
   __syncwarp();
 #pragma unroll
-  for (int k1 = 0; k1 < R; k1++) col[pidx(k1 * P + t)] = v[k1];
+  for (int k1 = 0; k1 < R; k1++) col[widx<T2>(k1 * P + t)] = v[k1];
   __syncwarp();
   if (P == R) {
 #pragma unroll
-    for (int m = 0; m < P; m++) v[m] = col[pidx(t * P + m)];
+    for (int m = 0; m < P; m++) v[m] = col[widx<T2>(t * P + m)];
     dft<P, T2, T>(v);
     __syncwarp();
 #pragma unroll
     for (int k2 = 0; k2 < P; k2++) {
       T2 o = v[k2];
       if (INV) o.y = -o.y;
-      col[pidx(t + R * k2)] = o;
+      col[widx<T2>(t + R * k2)] = o;
     }
   } else {  // P == 2R: threads (k1, h) hold the even (h = 0) / odd (h = 1) half
     const int k1 = t >> 1, hh = t & 1;
 #pragma unroll
-    for (int m = 0; m < R; m++) v[m] = col[pidx(k1 * P + 2 * m + hh)];
+    for (int m = 0; m < R; m++) v[m] = col[widx<T2>(k1 * P + 2 * m + hh)];
     dft<R, T2, T>(v);
     __syncwarp();
 #pragma unroll
@@ -141,7 +141,7 @@ __device__ __forceinline__ void column(T2* col, const T2* tw, int t) {
       o.x = hh ? e.x - w.x : e.x + w.x;
       o.y = hh ? e.y - w.y : e.y + w.y;
       if (INV) o.y = -o.y;
-      col[pidx(k1 + R * (hh * R + i))] = o;
+      col[widx<T2>(k1 + R * (hh * R + i))] = o;
     }
   }
   __syncwarp();

@@ -694,7 +694,19 @@ constexpr int ncols9() { return ((9 + cpw<N>() - 1) / cpw<N>()) * cpw<N>(); }
 template <int N, int TK>
 constexpr int ncols_c() { return ((9 * TK + cpw<N>() - 1) / cpw<N>()) * cpw<N>(); }
 
-// Transform ncols columns (stride Lp; ncols a multiple of cpw<N>()) with every warp of
+// Distance of pass C's columns: its tile moves TK columns side by side, so consecutive columns
+// start 16 / TK (8-byte elements) or 8 / TK (16-byte) elements apart modulo one bank sweep, and
+// the lanes of a sweep, TK columns by 16 / TK (8 / TK) neighbours along c, hit distinct banks.
+// Shared-memory sweeps bound the FP32 passes on the cached spectrum; with N + N/8 + 1 and k + k/8
+// everywhere an element cost 28 where it now costs 12 (128^3 FP32, a launch: C 103 to 77 us, B
+// 46 to 38, E 57 to 51).
+template <int N, typename T2, int TK>
+constexpr int stride_c() {
+  constexpr int W = 128 / (int)sizeof(T2), len = N + (N >> 3);
+  return len + (W / TK - len % W + W) % W;
+}
+
+// Transform ncols columns (stride Lp; rounded up to a multiple of cpw<N>()) with every warp of
 // the block; inverse through conjugation.  Columns past the data are scratch.
 template <int N, typename T, bool INV>
 __device__ __forceinline__ void block_columns(typename Vec2<T>::t* base, int ncols, int Lp,
@@ -776,8 +788,8 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, T>()) wpass_a(const TIO* 
     }
 #pragma unroll
     for (int i = 0; i < 9; i++) {
-      if (l == 0) col[i * Lp + pidx(a)].x = y[i];
-      else col[i * Lp + pidx(a)].y = y[i];
+      if (l == 0) col[i * Lp + widx<T2>(a)].x = y[i];
+      else col[i * Lp + widx<T2>(a)].y = y[i];
     }
   }
   if (part) block_partial<288>(to_io<double, T>(dsum), part + blockIdx.x);
@@ -786,7 +798,7 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, T>()) wpass_a(const TIO* 
   __syncthreads();
   for (int t = threadIdx.x; t < 9 * H; t += blockDim.x) {
     int i = t / H, k = t - i * H;
-    T2 z = col[i * Lp + pidx(k)], wv = conjg(col[i * Lp + pidx((N - k) & (N - 1))]);
+    T2 z = col[i * Lp + widx<T2>(k)], wv = conjg(col[i * Lp + widx<T2>((N - k) & (N - 1))]);
     T2 X0, X1;
     X0.x = (T)0.5 * (z.x + wv.x); X0.y = (T)0.5 * (z.y + wv.y);
     X1.x = (T)0.5 * (z.y - wv.y); X1.y = (T)-0.5 * (z.x - wv.x);
@@ -825,17 +837,18 @@ __global__ void __launch_bounds__(32 * TK / cpw<32 * M>()) wpass_b(typename Vec2
 #pragma unroll
     for (int e = 0; e < E; e++) {
       const int t = threadIdx.x + e * NT, row = t / TK, kk = t % TK;
-      col[kk * Lp + pidx(row)] = v[e];
+      col[kk * Lp + widx<T2>(row)] = v[e];
     }
   }
   __syncthreads();
-  if (inverse) block_columns<N, T, true>(col, TK, Lp, tw);
-  else block_columns<N, T, false>(col, TK, Lp, tw);
+  const int nc = min(TK, H - ka0);  // the last tile's missing columns are not transformed
+  if (inverse) block_columns<N, T, true>(col, nc, Lp, tw);
+  else block_columns<N, T, false>(col, nc, Lp, tw);
   __syncthreads();
   for (int t = threadIdx.x; t < TK * N; t += blockDim.x) {
     int row = t / TK, kk = t - row * TK;
     int ka = ka0 + kk;
-    if (ka < H) plane[(long long)row * H + ka] = col[kk * Lp + pidx(row)];
+    if (ka < H) plane[(long long)row * H + ka] = col[kk * Lp + widx<T2>(row)];
   }
 }
 
@@ -844,7 +857,7 @@ __global__ void __launch_bounds__(288) wpass_c(typename Vec2<T>::t* __restrict__
                                                const typename Vec2<T>::t* __restrict__ twg) {
   using T2 = typename Vec2<T>::t;
   constexpr int N = 32 * M, H = N / 2 + 1;
-  const int Lp = padlen(N);
+  constexpr int Lp = stride_c<N, T2, TK>();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   T2* tw = reinterpret_cast<T2*>(smem_raw);
   T2* col = tw + N;
@@ -869,7 +882,7 @@ __global__ void __launch_bounds__(288) wpass_c(typename Vec2<T>::t* __restrict__
     for (int e = 0; e < E; e++) {
       const int t = threadIdx.x + e * NT, kk = t % TK, rem = t / TK;
       const int c = rem % N, i = rem / N;
-      col[(i * TK + kk) * Lp + pidx(c)] = v[e];
+      col[(i * TK + kk) * Lp + widx<T2>(c)] = v[e];
     }
   }
   __syncthreads();
@@ -883,7 +896,7 @@ __global__ void __launch_bounds__(288) wpass_c(typename Vec2<T>::t* __restrict__
     T2 A[9], out[9];
 #pragma unroll
     for (int i = 0; i < 9; i++) {
-      A[i] = col[(i * TK + kk) * Lp + pidx(kc)];
+      A[i] = col[(i * TK + kk) * Lp + widx<T2>(kc)];
       out[i].x = 0; out[i].y = 0;
     }
     bool nyq = gm == CPFFT_G_CENTERED && (2 * kc == N || 2 * kb == N || 2 * ka == N);
@@ -899,7 +912,7 @@ __global__ void __launch_bounds__(288) wpass_c(typename Vec2<T>::t* __restrict__
       }
     }
 #pragma unroll
-    for (int i = 0; i < 9; i++) col[(i * TK + kk) * Lp + pidx(kc)] = out[i];
+    for (int i = 0; i < 9; i++) col[(i * TK + kk) * Lp + widx<T2>(kc)] = out[i];
   }
   __syncthreads();
   block_columns<N, T, true>(col, ncols_c<N, TK>(), Lp, tw);
@@ -909,7 +922,7 @@ __global__ void __launch_bounds__(288) wpass_c(typename Vec2<T>::t* __restrict__
     int c = rem % N, i = rem / N;
     int ka = ka0 + kk;
     if (ka < H)
-      S[((long long)i * N) * cstr + c * cstr + (long long)kb * H + ka] = col[(i * TK + kk) * Lp + pidx(c)];
+      S[((long long)i * N) * cstr + c * cstr + (long long)kb * H + ka] = col[(i * TK + kk) * Lp + widx<T2>(c)];
   }
 }
 
@@ -1125,7 +1138,7 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, T>()) wpass_e(const typen
       T2 z;  // Z = X0 + i X1 (the inverse is taken as conj(FFT(conj Z)))
       z.x = a.x - b.y;
       z.y = a.y + b.x;
-      col[i * Lp + pidx(k)] = z;
+      col[i * Lp + widx<T2>(k)] = z;
     }
   }
   // the other factor of the fused product, loaded before the transform hides its latency
@@ -1147,7 +1160,7 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, T>()) wpass_e(const typen
   for (int e = 0; e < EO; e++) {
     const int t = threadIdx.x + e * NT, l = t / (9 * N), rem = t - l * 9 * N;
     const int i = rem / N, a = rem - i * N;
-    T2 z = col[i * Lp + pidx(a)];  // unscaled inverse (scale applied in pass C)
+    T2 z = col[i * Lp + widx<T2>(a)];  // unscaled inverse (scale applied in pass C)
     long long v = a + (long long)N * (bl0 + l) + (long long)N * N * c;
     const T yv = l ? z.y : z.x;
     y[i * N3 + v] = to_io<TIO, T>(yv);
@@ -1213,7 +1226,7 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, float>()) wpass_e_xr(
       T2 z;  // Z = X0 + i X1 (the inverse is taken as conj(FFT(conj Z)))
       z.x = a.x - b.y;
       z.y = a.y + b.x;
-      col[i * Lp + pidx(k)] = z;
+      col[i * Lp + widx<T2>(k)] = z;
     }
   }
   float xv[NV][9], rv[NV][9], pv[NV][9];
@@ -1244,7 +1257,7 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, float>()) wpass_e_xr(
       const long long v = a + (long long)N * (bl0 + l) + (long long)N * N * c;
 #pragma unroll
       for (int i = 0; i < 9; i++) {
-        const T2 z = col[i * Lp + pidx(a)];  // unscaled inverse (scale applied in pass C)
+        const T2 z = col[i * Lp + widx<T2>(a)];  // unscaled inverse (scale applied in pass C)
         const float ap = l ? z.y : z.x;
         xv[u][i] += alpha * pv[u][i];
         rv[u][i] -= alpha * ap;
@@ -1265,6 +1278,12 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, float>()) wpass_e_xr(
 
 template <typename T>
 size_t smem_w(int N, int ncols) { return sizeof(typename Vec2<T>::t) * (size_t)(N + ncols * padlen(N)); }
+// pass C's shared memory
+template <typename T, int N, int TK>
+constexpr size_t smem_wc() {
+  using T2 = typename Vec2<T>::t;
+  return sizeof(T2) * (size_t)(N + ncols_c<N, TK>() * stride_c<N, T2, TK>());
+}
 template <typename T>
 constexpr int wtile_c() { return sizeof(T) == 4 ? 4 : 2; }
 
@@ -1276,8 +1295,8 @@ constexpr int TB_CAND[3] = {8, 16, 32};
 constexpr int TC_CAND[2] = {2, 4};
 // pass C in registers (wpass_c2, FP32 only): its TK.  The slowest-axis algorithm is fixed
 // per grid, because the two round differently and contexts of one grid must give identical
-// results whatever their timings: in registers up to N = 64 (64^3: 12.9 against 19.4 us a
-// launch), in shared memory above (128^3: 120 against 103 us), measured with ncu on a
+// results whatever their timings: in registers up to N = 64 (64^3: 12.9 against 18.7 us a
+// launch), in shared memory above (128^3: 121 against 77 us), measured with ncu on a
 // GB300; the autotuner then chooses the tiles within that algorithm.  cpfft_set_tiles
 // selects either.
 constexpr int C2_CAND[2] = {2, 4};
@@ -1293,7 +1312,7 @@ template <int M, typename T, int TC>
 cudaError_t wsetup_c() {
   constexpr int N = 32 * M;
   return cudaFuncSetAttribute(wpass_c<M, T, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              (int)smem_w<T>(N, ncols_c<N, TC>()));
+                              (int)smem_wc<T, N, TC>());
 }
 
 template <typename T>
@@ -1348,7 +1367,7 @@ void wlaunch_c(typename Vec2<T>::t* S, const GridDesc& g, const typename Vec2<T>
                cudaStream_t st) {
   constexpr int N = 32 * M, H = N / 2 + 1;
   dim3 gc((H + TC - 1) / TC, N);
-  wpass_c<M, T, TC><<<gc, 288, smem_w<T>(N, ncols_c<N, TC>()), st>>>(S, g, tw);
+  wpass_c<M, T, TC><<<gc, 288, smem_wc<T, N, TC>(), st>>>(S, g, tw);
 }
 template <int M, typename T>
 void wlaunch_b_any(int tb, typename Vec2<T>::t* S, const GridDesc& g,
