@@ -3,6 +3,8 @@
 // FP32 register passes) and green_df.cu (double-float register passes).  Each unit gets
 // its own copies in an unnamed namespace.
 #pragma once
+#include <type_traits>
+
 #include "fft_green.cuh"
 #include "fft_warp.cuh"
 #include "krylov.cuh"
@@ -718,22 +720,30 @@ __device__ __forceinline__ void block_columns(typename Vec2<T>::t* base, int nco
     regfft::column<N, T2, T, INV>(base + (g * CPW + lane / P) * Lp, tw, lane % P);
 }
 
-// part != nullptr (with flgK): one partial sum per block of <K : x, x> over its voxels.
-// Resident blocks per SM the FP32 passes A and E are compiled for at N = 128: four
-// 288-thread blocks (at most 56 registers a thread) keep more loads in flight than the
-// three the default register count allows -- 5 % off the FP32 apply at 128^3, measured.
-// 0 (no hint) elsewhere: the double-float passes, N = 256 (the cap would spill) and the
-// small grids (whose default counts already fit more blocks).
+// Threads of passes A and E.  Their 9 lines fill 5 warps of the transform at P = 16 and 3 at P = 8:
+// blocks of 6 and 3 warps leave few warps idle in it, where the arithmetic of the 16-byte types
+// spends its time.  Double-float apply, 288 threads against these: 32^3 53.7 to 45.3 us, 64^3 280
+// to 265 us, 128^3 1.28 to 1.24 ms, 256^3 13.4 to 11.6 ms.  FP32 keeps 288 (more loads in flight).
 template <int M, typename T>
-constexpr int minblocks_ae() { return (sizeof(T) == 4 && M == 4) ? 4 : 0; }
+constexpr int ae_threads() {
+  return sizeof(T) == 4 ? 288 : regfft::Shape<32 * M>::P == 16 ? 192 : 96;
+}
+// Resident blocks per SM passes A and E are compiled for at N = 128, four: FP32 (288 threads, at
+// most 56 registers) keeps more loads in flight than the three the default register count
+// allows -- 5 % off the FP32 apply at 128^3, measured -- and double-float (192 threads) has 20
+// transforming warps instead of 15 (apply 1.31 to 1.24 ms).  0 (no hint) elsewhere: FP64, N = 256
+// (no gain, FP32 would spill) and the small grids (whose default counts already fit more blocks).
+template <int M, typename T>
+constexpr int minblocks_ae() { return M == 4 && !std::is_same<T, double>::value ? 4 : 0; }
 
+// part != nullptr (with flgK): one partial sum per block of <K : x, x> over its voxels.
 // TIO: the field type of x (float, or double for the double-float transform T = dfl,
 // whose tangent is the pair K4, K4lo)
 // FUSEP (FP32 CG iteration): the operand is the CG direction updated in place on load,
 // p = r + beta p with beta = sc[SC_BETA] (x is p, rfuse is r), and sc[SC_RR] takes
 // sc[SC_RRNEW] -- the work of k_cg_p fused into this pass.
 template <int M, typename T, typename TK, typename TIO, bool FUSEP = false>
-__global__ void __launch_bounds__(288, minblocks_ae<M, T>()) wpass_a(const TIO* __restrict__ x, const TK* __restrict__ K4,
+__global__ void __launch_bounds__(ae_threads<M, T>(), minblocks_ae<M, T>()) wpass_a(const TIO* __restrict__ x, const TK* __restrict__ K4,
                                                const float* __restrict__ K4lo,
                                                int flgK, typename Vec2<T>::t* __restrict__ S,
                                                GridDesc g, const typename Vec2<T>::t* __restrict__ twg,
@@ -792,7 +802,7 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, T>()) wpass_a(const TIO* 
       else col[i * Lp + widx<T2>(a)].y = y[i];
     }
   }
-  if (part) block_partial<288>(to_io<double, T>(dsum), part + blockIdx.x);
+  if (part) block_partial<ae_threads<M, T>()>(to_io<double, T>(dsum), part + blockIdx.x);
   __syncthreads();
   block_columns<N, T, false>(col, ncols9<N>(), Lp, tw);
   __syncthreads();
@@ -1101,7 +1111,7 @@ __global__ void __launch_bounds__(c2_threads<32 * M, TK>()) wpass_c2(
 // dotx != nullptr: also one partial sum per block of dotx . y over the voxels the block
 // writes (the CG product p . Ap without re-reading Ap), into part[blockIdx.x]
 template <int M, typename T, typename TIO>
-__global__ void __launch_bounds__(288, minblocks_ae<M, T>()) wpass_e(const typename Vec2<T>::t* __restrict__ S,
+__global__ void __launch_bounds__(ae_threads<M, T>(), minblocks_ae<M, T>()) wpass_e(const typename Vec2<T>::t* __restrict__ S,
                                                TIO* __restrict__ y, GridDesc g,
                                                const typename Vec2<T>::t* __restrict__ twg,
                                                const TIO* __restrict__ dotx,
@@ -1116,7 +1126,7 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, T>()) wpass_e(const typen
   load_tw(tw, twg, N);
   const int bp = blockIdx.x % (N / 2), c = blockIdx.x / (N / 2);
   const int bl0 = 2 * bp;
-  constexpr int NT = 288, E = 9 * N / NT;
+  constexpr int NT = ae_threads<M, T>(), E = 9 * N / NT;
   static_assert(E * NT == 9 * N, "lines must divide evenly over the block");
   {
     T2 X0[E], X1[E];
@@ -1166,15 +1176,15 @@ __global__ void __launch_bounds__(288, minblocks_ae<M, T>()) wpass_e(const typen
     y[i * N3 + v] = to_io<TIO, T>(yv);
     if (dotx) dsum += px[e] * yv;
   }
-  if (dotx) {  // block sum (9 warps), fixed order
-    __shared__ double wsum[9];
+  if (dotx) {  // block sum, fixed order
+    __shared__ double wsum[NT / 32];
     double d = to_io<double, T>(dsum);
     for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
     if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = d;
     __syncthreads();
     if (threadIdx.x == 0) {
       double b = 0.0;
-      for (int k = 0; k < 9; k++) b += wsum[k];
+      for (int k = 0; k < NT / 32; k++) b += wsum[k];
       part[blockIdx.x] = b;
     }
   }
@@ -1392,13 +1402,13 @@ void wgreen_apply(const TIO* x, const TK* K4, const float* K4lo, int flgK, TIO* 
   double* part_e = g.pre ? nullptr : part;
   if constexpr (small_code<T>()) {
     if (rfuse)
-      wpass_a<M, T, TK, TIO, true><<<(N / 2) * N, 288, smem_w<T>(N, NA), st>>>(
+      wpass_a<M, T, TK, TIO, true><<<(N / 2) * N, ae_threads<M, T>(), smem_w<T>(N, NA), st>>>(
           x, K4, K4lo, flgK, S, g, tw, part_a, rfuse, scf, const_cast<TIO*>(x));
     else
-      wpass_a<M, T, TK, TIO><<<(N / 2) * N, 288, smem_w<T>(N, NA), st>>>(x, K4, K4lo, flgK, S, g,
+      wpass_a<M, T, TK, TIO><<<(N / 2) * N, ae_threads<M, T>(), smem_w<T>(N, NA), st>>>(x, K4, K4lo, flgK, S, g,
                                                                         tw, part_a);
   } else {
-    wpass_a<M, T, TK, TIO><<<(N / 2) * N, 288, smem_w<T>(N, NA), st>>>(x, K4, K4lo, flgK, S, g, tw,
+    wpass_a<M, T, TK, TIO><<<(N / 2) * N, ae_threads<M, T>(), smem_w<T>(N, NA), st>>>(x, K4, K4lo, flgK, S, g, tw,
                                                                       part_a);
   }
   wlaunch_b_any<M, T>(g.wtb, S, g, tw, 0, st);
@@ -1411,7 +1421,7 @@ void wgreen_apply(const TIO* x, const TK* K4, const float* K4lo, int flgK, TIO* 
     wlaunch_c<M, T, 2>(S, g, tw, st);
   }
   wlaunch_b_any<M, T>(g.wtb, S, g, tw, 1, st);
-  wpass_e<M, T, TIO><<<(N / 2) * N, 288, smem_w<T>(N, NA), st>>>(S, y, g, tw,
+  wpass_e<M, T, TIO><<<(N / 2) * N, ae_threads<M, T>(), smem_w<T>(N, NA), st>>>(S, y, g, tw,
                                                                  part_e ? x : nullptr, part_e);
 }
 
