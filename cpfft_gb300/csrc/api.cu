@@ -488,8 +488,8 @@ struct Ctx {
   // reference-medium preconditioner of the FP32 inner iterations (cpfft_set_precond)
   int precond = 0;
   bool pre_ok = false;     // the current reference medium is usable
-  double* k0sum = nullptr; // (81) component sums of K4f
-  double* h_k0 = nullptr;  // pinned (81) copy
+  double* k0sum = nullptr; // (81) component sums of K4f, then dev_medium's rows
+  double* h_k0 = nullptr;  // pinned copy
   float* h_pre = nullptr;  // pinned: 36 acoustic coefficients + 81 entries of K0
   float* pre_dev = nullptr;  // the same on the device (read by the preconditioned kernels)
   // FFT_nr3 locals that persist across steps (Fortran DATA => SAVE, src/FFT_nr3.f:29-34)
@@ -724,21 +724,23 @@ int matvec32_alpha(Ctx* c, const float* x, float* y) {
 // <a, b>_K0 on compatible fields, where CG on it is CG preconditioned by G(K0 : .).  Its
 // iteration count follows the contrast of K against K0 instead of against the identity.
 
-// Sums of K4f (after a stress update or an uploaded tangent), read back with the stream's
-// next synchronisation; reference_build then forms the medium.
+// Sums of K4f (after a stress update or an uploaded tangent) and the medium's ellipticity,
+// read back with the stream's next synchronisation; reference_build then forms the medium.
 int reference_reduce(Ctx* c) {
   if (!c->k0sum) {
-    TRY(dalloc(c->k0sum, 81 * sizeof(double)));
+    TRY(dalloc(c->k0sum, (81 + MEDIUM_ROWS) * sizeof(double)));
     TRY(dalloc(c->pre_dev, (36 + 81) * sizeof(float)));
     c->g.acoef = c->pre_dev;
-    if (cudaMallocHost((void**)&c->h_k0, 81 * sizeof(double)) != cudaSuccess ||
+    if (cudaMallocHost((void**)&c->h_k0, (81 + MEDIUM_ROWS) * sizeof(double)) != cudaSuccess ||
         cudaMallocHost((void**)&c->h_pre, (36 + 81) * sizeof(float)) != cudaSuccess) {
       cpfft_set_error("cudaMallocHost failed");
       return CPFFT_ERR_NO_MEMORY;
     }
   }
   CK(dev_mean81(c->K4f, c->N3, c->part, c->k0sum, c->st));
-  CK(cudaMemcpyAsync(c->h_k0, c->k0sum, 81 * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+  CK(dev_medium(c->k0sum, c->N3, c->k0sum + 81, c->st));
+  CK(cudaMemcpyAsync(c->h_k0, c->k0sum, (81 + MEDIUM_ROWS) * sizeof(double),
+                     cudaMemcpyDeviceToHost, c->st));
   return 0;
 }
 
@@ -764,28 +766,9 @@ int reference_build(Ctx* c) {
       if (j != l) v += K0[9 * (3 * i + l) + 3 * k + j];
       coef[6 * r + m] = v;
     }
-  // positive definiteness (Sylvester) with a margin, on 64 x 128 directions of the sphere
-  const double pi = 3.14159265358979323846;
-  double lo = 1e300, hi = 0.0;
-  for (int it = 0; it <= 64; it++)
-    for (int ip = 0; ip < 128; ip++) {
-      const double th = pi * it / 64.0, ph = 2.0 * pi * ip / 128.0;
-      const double n[3] = {std::sin(th) * std::cos(ph), std::sin(th) * std::sin(ph), std::cos(th)};
-      const double pr[6] = {n[0] * n[0], n[1] * n[1], n[2] * n[2], n[0] * n[1], n[1] * n[2], n[0] * n[2]};
-      double a[6];
-      for (int r = 0; r < 6; r++) {
-        a[r] = 0.0;
-        for (int m = 0; m < 6; m++) a[r] += coef[6 * r + m] * pr[m];
-      }
-      const double m2 = a[0] * a[1] - a[3] * a[3];
-      const double det = a[0] * (a[1] * a[2] - a[4] * a[4]) - a[3] * (a[3] * a[2] - a[4] * a[5]) +
-                         a[5] * (a[3] * a[4] - a[1] * a[5]);
-      const double tr = a[0] + a[1] + a[2];
-      if (!(a[0] > 0.0 && m2 > 0.0 && det > 0.0 && tr > 0.0)) return 0;
-      // det / tr^3 bounds the smallest eigenvalue's share from below
-      lo = std::min(lo, det / (tr * tr * tr));
-      hi = std::max(hi, tr);
-    }
+  double lo = c->h_k0[81];
+  for (int k = 1; k < MEDIUM_ROWS; k++) lo = std::min(lo, c->h_k0[81 + k]);
+  if (!(lo > 0.0)) return 0;
   if (c->log)
     fprintf(stderr, "         reference medium: min det/tr^3 of the acoustic tensor %.3e%s\n", lo,
             lo > 1.0e-9 ? "" : " (not used)");

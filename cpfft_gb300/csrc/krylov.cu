@@ -334,6 +334,58 @@ __global__ void __launch_bounds__(64) k_final_rows(const double* __restrict__ pa
   if (threadIdx.x == 0) out[blockIdx.x] = ws[0] + ws[1];
 }
 
+// Ellipticity of the reference medium K0 = sym(sums / N3) / its largest entry: the acoustic
+// tensor A(n)_ik = K0_ijkl n_j n_l on MEDIUM_ROWS x 128 directions of the sphere, one a thread;
+// out[b] = the least det A / tr(A)^3 of block b's directions (it bounds the smallest
+// eigenvalue's share from below), -1 where A is not positive definite (Sylvester).  On the host
+// the 8,320 directions held up every stress pass of the fast form with the GPU idle; here they
+// run between the sums and their read-back (a 12^3 pass 1.17 to 0.95 ms, a 62^3 one 8.16 to
+// 7.98).
+__global__ void __launch_bounds__(128) k_medium(const double* __restrict__ sc81, long long N3,
+                                                double* __restrict__ out) {
+  __shared__ double K0[81], wmin[4], s_mx;
+  const int t = threadIdx.x;
+  if (t < 81) K0[t] = 0.5 * (sc81[t] + sc81[9 * (t % 9) + t / 9]) / (double)N3;
+  __syncthreads();
+  if (t < 32) {
+    double m = fmax(fabs(K0[t]), fabs(K0[t + 32]));
+    if (t + 64 < 81) m = fmax(m, fabs(K0[t + 64]));
+    for (int o = 16; o > 0; o >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if (t == 0) s_mx = m;
+  }
+  __syncthreads();
+  if (t < 81) K0[t] /= s_mx;
+  __syncthreads();
+  double n[3], sth, cth, sph, cph;
+  sincospi(blockIdx.x / (double)(MEDIUM_ROWS - 1), &sth, &cth);
+  sincospi(t / 64.0, &sph, &cph);
+  n[0] = sth * cph; n[1] = sth * sph; n[2] = cth;
+  double a[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      a[i][k] = 0.0;
+#pragma unroll
+      for (int j = 0; j < 3; j++) {
+        double v = 0.0;
+#pragma unroll
+        for (int l = 0; l < 3; l++) v += K0[9 * (3 * i + j) + 3 * k + l] * n[l];
+        a[i][k] += v * n[j];
+      }
+    }
+  const double m2 = a[0][0] * a[1][1] - a[0][1] * a[0][1];
+  const double det = a[0][0] * (a[1][1] * a[2][2] - a[1][2] * a[1][2]) -
+                     a[0][1] * (a[0][1] * a[2][2] - a[1][2] * a[0][2]) +
+                     a[0][2] * (a[0][1] * a[1][2] - a[1][1] * a[0][2]);
+  const double tr = a[0][0] + a[1][1] + a[2][2];
+  double q = a[0][0] > 0.0 && m2 > 0.0 && det > 0.0 && tr > 0.0 ? det / (tr * tr * tr) : -1.0;
+  for (int o = 16; o > 0; o >>= 1) q = fmin(q, __shfl_xor_sync(0xffffffffu, q, o));
+  if ((t & 31) == 0) wmin[t >> 5] = q;
+  __syncthreads();
+  if (t == 0) out[blockIdx.x] = fmin(fmin(wmin[0], wmin[1]), fmin(wmin[2], wmin[3]));
+}
+
 // The iteration graph's first node: its WHILE loop runs only if the iterations are not
 // already stopped (an eager first iteration may have met the stop test), so the host
 // launches the graph without reading the stop flag first.
@@ -477,6 +529,10 @@ cudaError_t dev_mean81(const float* K, long long N3, double* part, double* sc81,
   k_sum81<<<dim3(NB, 81), RB, 0, st>>>(K, N3, part);
   k_final_rows<<<81, 64, 0, st>>>(part, NB, sc81);
   return counted(2);
+}
+cudaError_t dev_medium(const double* sc81, long long N3, double* out, cudaStream_t st) {
+  k_medium<<<MEDIUM_ROWS, 128, 0, st>>>(sc81, N3, out);
+  return counted(1);
 }
 cudaError_t dev_cg_gate(const double* sc, cudaGraphConditionalHandle h, cudaStream_t st) {
   k_cg_gate<<<1, 1, 0, st>>>(sc, h);

@@ -73,6 +73,10 @@ cudaError_t dev_dot_k0(const float* a, const float* b, long long N3, const float
                        double* part, double* sc, int slot, int op, cudaStream_t st);
 // sc81[m] = sum over voxels of component m of an (81, N3) FP32 field (part: 81 x 64)
 cudaError_t dev_mean81(const float* K, long long N3, double* part, double* sc81, cudaStream_t st);
+// least det / tr^3 of the acoustic tensor of the sums' mean over each row of directions, -1
+// where it is not positive definite
+constexpr int MEDIUM_ROWS = 65;  // polar angles, 128 directions each
+cudaError_t dev_medium(const double* sc81, long long N3, double* out, cudaStream_t st);
 
 // End-of-iteration test of a preconditioned FP32 CG segment (cg_cond, one thread, with
 // OP_BETA_COND): counts the iteration and stops when the K0 norm of the residual has dropped by
