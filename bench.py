@@ -58,7 +58,7 @@ BYTES_CG32_FUSED = 756.0
 # FP64 flops of a stress pass per voxel (2 DFMA + DADD + DMUL of active lanes, ncu at 64^3):
 # explicit passes (iteration 0), and implicit passes as a base plus a cost per local Newton
 # iteration (predictor iterations included), fitted over one timed load step's passes
-STRESS_FLOPS = {"explicit": 3933.0, "implicit_base": 6433.0, "per_iteration": 3909.0,
+STRESS_FLOPS = {"explicit": 3933.0, "implicit_base": 5195.0, "per_iteration": 2912.0,
                 "source": "profiles/stress_kernel_64.md (ncu FP64 instruction counts of 8 "
                           "passes at 64^3, fitted to their local iterations)"}
 FUSED_GRIDS = (32, 64, 128, 256)

@@ -236,6 +236,7 @@ int cpfft_set_schedule(int schedule);
  * CPFFT_SCHED_QUEUE pass the pass runs once per candidate -- 128, 256 or 512 voxels taken
  * from the queue by a block at a time, with as many persistent blocks per SM as fit or
  * with one -- timed with CUDA events, and the fastest is kept (identical results).
+ * Passes of the dislocation-density laws take the voxels in order and choose nothing.
  * *voxels = the chosen chunk (0 before that pass); *blocks_per_sm = 0 (as many as fit) or
  * 1; ms (6, may be NULL) = the pass times of the candidates, chunks 128 / 256 / 512 with
  * all blocks, then with one block per SM. */
