@@ -180,11 +180,15 @@ cudaError_t green_setup(int N) {
   if ((e = raise_max_dynamic_smem((const void*)pass_b<T>, b))) return e;
   if ((e = raise_max_dynamic_smem((const void*)pass_c<T>, c))) return e;
   if ((e = raise_max_dynamic_smem((const void*)pass_e<T>, a))) return e;
-  {
+  // the three-pass kernels run up to small_max only; a plane of a larger grid outgrows a block
+  // (FP64: from 112^3 on)
+  if (N <= small_max<T>()) {
     const size_t sm = smem_small<T>(N);
     if ((e = raise_max_dynamic_smem((const void*)small_forward<T, false>, sm))) return e;
     if ((e = raise_max_dynamic_smem((const void*)small_inverse<T, false>, sm))) return e;
-    if ((e = raise_max_dynamic_smem((const void*)small_columns<false>, smem_small<double>(N)))) return e;
+    if constexpr (sizeof(T) == 8) {
+      if ((e = raise_max_dynamic_smem((const void*)small_columns<false>, sm))) return e;
+    }
   }
   return cudaSuccess;
 }
