@@ -1,9 +1,6 @@
 // api.cu -- the C-ABI of include/cpfft_gpu.h: device context, material set-up, and the
 // host-side control of the resident Newton-Krylov loop (FFT_nr3 / fftPcg /
 // tangent_homo / NBC_update of src/FFT_nr3.f and src/tangent_homo.f).
-#include <sys/mman.h>
-#include <unistd.h>
-
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -39,6 +36,7 @@ bool mlp_device_weights(mlp::Weights* w, int** err);
 int mlp_check_error();
 #include "krylov.cuh"
 #include "cg_small.cuh"
+#include "prefault.hpp"
 
 // per host thread: a thread drives one context (cpfft_batch_solve runs several at once)
 static thread_local char g_err[512] = "";
@@ -554,38 +552,6 @@ void kt_reset(Ctx* c) {
   for (int k = 0; k < 4; k++) { c->kt_acc[k] = 0; c->kt_cnt[k] = 0; }
 }
 thread_local Ctx* g_ctx = nullptr;
-
-// Pages of large host output buffers made present by helper threads while the GPU works: a
-// device-to-host copy into untouched pages faults them one by one (151 MB: 5.5 ms against
-// 0.8 ms into present pages; two to four threads prepare them in 1.8 ms).  Contents are
-// kept; a buffer the call cannot prepare is left to the copy.
-class Prefault {
-  std::vector<std::thread> th_;
-
- public:
-  Prefault(std::initializer_list<std::pair<void*, size_t>> bufs) {
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    for (const auto& b : bufs) {
-      const size_t a0 = ((size_t)b.first + page - 1) / page * page;
-      const size_t a1 = ((size_t)b.first + b.second) / page * page;
-      if (!b.first || b.second < (4u << 20) || a1 <= a0) continue;
-      const size_t nt = std::min<size_t>(4, (a1 - a0) >> 22), part = (a1 - a0) / (nt * page) * page;
-      for (size_t k = 0; k < nt && part; k++) {
-        const size_t p0 = a0 + k * part, p1 = k + 1 == nt ? a1 : p0 + part;
-        try {
-          th_.emplace_back([p0, p1] { madvise((void*)p0, p1 - p0, 23 /* MADV_POPULATE_WRITE */); });
-        } catch (...) {  // no thread to be had: the copy faults the pages itself
-          return;
-        }
-      }
-    }
-  }
-  void join() {
-    for (auto& t : th_) t.join();
-    th_.clear();
-  }
-  ~Prefault() { join(); }
-};
 
 #define TRY(expr)                 \
   do {                            \
