@@ -342,24 +342,6 @@ void mrr_interaction(int slip_type, double Gm[144], double Hm[144]) {
     }
 }
 
-// the table of x^y (PowTab); entries rounded once from long double
-bool pow_table(double y, PowTab& t) {
-  if (!(y > 0.0 && y <= 8.0)) return false;
-  t.y = y;
-  long double b = 1.0L;
-  for (int k = 1; k <= 6; k++) {
-    b *= ((long double)y - (k - 1)) / k;
-    t.c[k - 1] = (double)b;
-  }
-  for (int i = 0; i < PowTab::NM; i++) {
-    t.rc[i] = (double)(1.0L / (1.0L + (i + 0.5L) / PowTab::NM));
-    t.P[i] = (double)powl((long double)t.rc[i], -(long double)y);
-  }
-  // 2^(y k), infinite or zero past the exponent range as x^y is
-  for (int k = 0; k < PowTab::NE; k++) t.E[k] = (double)exp2l((long double)y * (k - PowTab::EMID));
-  return true;
-}
-
 CrysRec crystal_record(const cpfft_crystal& p) {
   CrysRec c;
   std::memset(&c, 0, sizeof(c));

@@ -5,6 +5,7 @@
 #include <cstdio>
 
 #include "../../include/cpfft_gpu.h"
+#include "powtab.hpp"
 
 #define CPFFT_CUDA_TRY(expr)                                                       \
   do {                                                                             \
@@ -35,17 +36,6 @@ struct OriRec {
   double ms[48 * 6];  // nslip x 6 sym(b (x) n) Voigt, engineering shear
   double qs[48 * 3];  // nslip x 3 skew(b (x) n) as (w23, w13, w12)
   double g[9];     // lattice -> sample rotation applied to b and n, row-major
-};
-
-// Table of x^y for a fixed exponent 0 < y <= 8 (tpow, stress.cu; filled by pow_table,
-// api.cu): x = 2^k m, c the midpoint of m's interval of [1, 2).
-struct PowTab {
-  static constexpr int NM = 256, NE = 1024, EMID = 512;
-  double y;
-  double c[6];     // binomial coefficients y, y (y - 1) / 2, .. of (1 + u)^y - 1
-  double rc[NM];   // 1 / c, rounded
-  double P[NM];    // rc^-y
-  double E[NE];    // 2^(y (k - EMID))
 };
 
 // Scalars of one crystal definition that the Voce path reads.

@@ -55,23 +55,6 @@ __device__ __forceinline__ double ipow(double x, int e) {
   }
   return r;
 }
-// x^y, x >= 0, with the exponent's table: x = 2^k m, the interval's 1/c from m's leading bits,
-// u = m / c - 1 (one rounding), c^y 2^(y k) ((1 + u)^y by its binomial series, |u| <= 2^-9).
-// Nine FP64 instructions where CUDA's pow takes about 95; error at most 2.5 ulp over the table's
-// range (0 < y <= 8, 2^-512 <= x < 2^512; pow elsewhere).
-__device__ __forceinline__ double tpow(const PowTab* __restrict__ t, double x) {
-  const int hi = __double2hiint(x);
-  const unsigned k = (unsigned)((hi >> 20) - 1023 + PowTab::EMID);
-  if (k >= PowTab::NE) return x == 0.0 ? 0.0 : pow(x, t->y);
-  const int i = (hi >> 12) & (PowTab::NM - 1);
-  const double m = __hiloint2double((hi & 0xfffff) | 0x3ff00000, __double2loint(x));
-  const double u = fma(m, __ldg(t->rc + i), -1.0);
-  const double w = __ldg(t->P + i) * __ldg(t->E + k);
-  double q = __ldg(t->c + 5);
-#pragma unroll
-  for (int j = 4; j >= 0; j--) q = fma(q, u, __ldg(t->c + j));
-  return fma(w, q * u, w);
-}
 // |x|^(n-1) and x^n (x > 0) for the crystal's rate exponent n
 __device__ __forceinline__ double pow_n1(const CrysRec& c, double x) {
   x = fabs(x);
