@@ -36,6 +36,7 @@ bool mlp_device_weights(mlp::Weights* w, int** err);
 int mlp_check_error();
 #include "krylov.cuh"
 #include "cg_small.cuh"
+#include "kept.hpp"
 #include "prefault.hpp"
 
 // per host thread: a thread drives one context (cpfft_batch_solve runs several at once)
@@ -2866,18 +2867,23 @@ int cpfft_f2disp(double lx, double ly, double lz, double* u) {
   }
   const int N = c->N;
   const long long N1 = N + 1, nodes = N1 * N1 * N1;
-  if (!c->dct_tab) {  // cos(pi k i / N), from the N + 1 distinct values; kept by the context
-    std::vector<double> cv(N1), ctab(N1 * N1);
-    for (long long m = 0; m < N1; m++) cv[m] = (double)cosl(3.14159265358979323846264338327950288L * m / N);
-    for (long long k = 0; k < N1; k++)
-      for (long long i = 0; i < N1; i++) {
-        const long long m = (k * i) % (2LL * N);
-        ctab[k * N1 + i] = cv[m <= N ? m : 2LL * N - m];
-      }
-    TRY(dalloc(c->dct_tab, ctab.size() * sizeof(double)));
-    CK(cudaMemcpyAsync(c->dct_tab, ctab.data(), ctab.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
-    TRY(sync(c));
-  }
+  // cos(pi k i / N), from the N + 1 distinct values; kept by the context
+  std::vector<double> ctab;
+  TRY(keep_filled(
+      c->dct_tab, [&](double*& p) { return dalloc(p, N1 * N1 * sizeof(double)); },
+      [&](double* p) {
+        std::vector<double> cv(N1);
+        for (long long m = 0; m < N1; m++) cv[m] = (double)cosl(3.14159265358979323846264338327950288L * m / N);
+        ctab.resize(N1 * N1);
+        for (long long k = 0; k < N1; k++)
+          for (long long i = 0; i < N1; i++) {
+            const long long m = (k * i) % (2LL * N);
+            ctab[k * N1 + i] = cv[m <= N ? m : 2LL * N - m];
+          }
+        CK(cudaMemcpyAsync(p, ctab.data(), ctab.size() * sizeof(double), cudaMemcpyHostToDevice, c->st));
+        return sync(c);
+      },
+      [](double* p) { cudaFree(p); }));
   // scratch: the CG's fields, which hold nothing between calls (a nodal field has
   // 3 (N + 1)^3 <= 9 N^3 values from N = 3 on)
   double *work = c->r, *du = c->p, *small = nullptr;
