@@ -1118,12 +1118,12 @@ int cg_mixed_pre(Ctx* c, const double* b, double* x, double tol, int* iters, boo
   for (;;) {
     // one segment of iterations on the device: until <r,r>_K0 has dropped by delta, the
     // true residual it predicts meets the stop test, or maxIter; then the reliable update,
-    // x += G(xf / scale) in FP64-accurate arithmetic and the true residual, enqueued behind it:
-    // the host waits once for both
+    // x += G(xf / scale) in FP64-accurate arithmetic (nothing after a non-finite segment) and the
+    // true residual, enqueued behind it: the host waits once for both
     int stop = 0, done = 0;
     TRY(cg_segment(c, rn, tolb, tola, delta, it, maxIter, rrk2, &done));
     restarts++;
-    CK(dev_take_f32(c->w2, c->xf, 1.0 / scale, n, c->st));
+    CK(dev_take_f32(c->w2, c->xf, 1.0 / scale, n, c->sc, c->st));
     TRY(matvec_acc(c, c->w2, c->Ap, 0));
     CK(dev_axpy(x, c->Ap, 1.0, n, c->st));
     TRY(matvec_acc(c, x, c->Ap, 1));

@@ -143,11 +143,13 @@ __global__ void k_add_const(double* __restrict__ y, double v, long long n) {
        i += (long long)gridDim.x * blockDim.x)
     y[i] += v;
 }
-// y = s * (double)x_f, x_f = 0
-__global__ void k_take_f32(double* __restrict__ y, float* __restrict__ x, double s, long long n) {
+// y = s * (double)x_f, or zero after a segment that ended on a non-finite value; x_f = 0
+__global__ void k_take_f32(double* __restrict__ y, float* __restrict__ x, double s, long long n,
+                           const double* __restrict__ sc) {
+  const bool drop = sc[SC_STOP] == (double)STOP_NONFINITE;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n;
        i += (long long)gridDim.x * blockDim.x) {
-    y[i] = s * (double)x[i];
+    y[i] = drop ? 0.0 : s * (double)x[i];
     x[i] = 0.0f;
   }
 }
@@ -482,8 +484,9 @@ cudaError_t dev_add_f32(double* y, const float* x, double s, long long n, cudaSt
   k_add_f32<<<grid_for(n, 256), 256, 0, st>>>(y, x, s, n);
   return counted(1);
 }
-cudaError_t dev_take_f32(double* y, float* x, double s, long long n, cudaStream_t st) {
-  k_take_f32<<<grid_for(n, 256), 256, 0, st>>>(y, x, s, n);
+cudaError_t dev_take_f32(double* y, float* x, double s, long long n, const double* sc,
+                         cudaStream_t st) {
+  k_take_f32<<<grid_for(n, 256), 256, 0, st>>>(y, x, s, n, sc);
   return counted(1);
 }
 cudaError_t dev_restart_f32(float* y, const double* x, double s, float* p, float k, long long n,

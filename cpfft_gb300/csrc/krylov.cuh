@@ -50,9 +50,11 @@ cudaError_t dev_add_f32(double* y, const float* x, double s, long long n, cudaSt
 cudaError_t dev_sum9(const double* x, long long N3, double* part, double* sc, int slot0,
                      cudaStream_t st);
 
-// The reliable update's vector work: y = s x with x cleared; y = s x (FP32) with p scaled by
-// k; y = a - b with sc[slot] = sum of y^2
-cudaError_t dev_take_f32(double* y, float* x, double s, long long n, cudaStream_t st);
+// The reliable update's vector work: y = s x with x cleared (y = 0 when sc[SC_STOP] says that the
+// segment ended on a non-finite value: the solution stays as it was); y = s x (FP32) with p scaled
+// by k; y = a - b with sc[slot] = sum of y^2
+cudaError_t dev_take_f32(double* y, float* x, double s, long long n, const double* sc,
+                         cudaStream_t st);
 cudaError_t dev_restart_f32(float* y, const double* x, double s, float* p, float k, long long n,
                             cudaStream_t st);
 cudaError_t dev_sub_norm(double* y, const double* a, const double* b, long long n, double* part,
