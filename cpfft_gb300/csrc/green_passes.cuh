@@ -723,10 +723,13 @@ __device__ __forceinline__ void block_columns(typename Vec2<T>::t* base, int nco
 // Threads of passes A and E.  Their 9 lines fill 5 warps of the transform at P = 16 and 3 at P = 8:
 // blocks of 6 and 3 warps leave few warps idle in it, where the arithmetic of the 16-byte types
 // spends its time.  Double-float apply, 288 threads against these: 32^3 53.7 to 45.3 us, 64^3 280
-// to 265 us, 128^3 1.28 to 1.24 ms, 256^3 13.4 to 11.6 ms.  FP32 keeps 288 (more loads in flight).
+// to 265 us, 128^3 1.28 to 1.24 ms, 256^3 13.4 to 11.6 ms.  Native FP64, passes A + E (ncu): 128^3
+// 1.44 ms either way, 256^3 13.0 to 11.2 ms, but 64^3 174 to 184 us, so that one keeps 288 (pass
+// A loads its tangent with three times the threads), as FP32 does (more loads in flight).
 template <int M, typename T>
 constexpr int ae_threads() {
-  return sizeof(T) == 4 ? 288 : regfft::Shape<32 * M>::P == 16 ? 192 : 96;
+  if (sizeof(T) == 4 || (M == 2 && std::is_same<T, double>::value)) return 288;
+  return regfft::Shape<32 * M>::P == 16 ? 192 : 96;
 }
 // Resident blocks per SM passes A and E are compiled for at N = 128, four: FP32 (288 threads, at
 // most 56 registers) keeps more loads in flight than the three the default register count
