@@ -228,7 +228,7 @@ cudaError_t cg_small_solve(const double* b, double* x, double* r, double* p, dou
                            cudaStream_t st) {
   SmallCg a{x, r, {p, p2}, Ap, b, K4, S, tw, g, part, sc, bar, tol, max_iter};
   // split stages while the butterflies' depth is what a phase waits for: 11^3 42 against
-  // 53 us an iteration, 13^3 57 / 67, but 12^3 39 / 35 and 17^3 94 / 49
+  // 53 us an iteration, 13^3 58 / 67, but 12^3 37 / 36, 16^3 43 / 42 and 20^3 81 / 59
   if (g.N <= 11 || g.N == 13) {
     a.g.plan = split_plan(g.N);
     return launch_small<true>(a, st);

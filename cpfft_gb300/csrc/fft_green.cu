@@ -57,18 +57,16 @@ FftPlan make_plan(int N) {
   return p;
 }
 
-// Threads per block of the shared-memory passes.  A stage has (columns x N / radix)
-// butterflies -- 81 to 162 for the radices 7 to 9 at N = 63 -- so 256 threads leave half of
-// the block idle while its registers (about 112 a thread in FP64) hold back other blocks;
-// below these sizes the grid does not fill the SMs and the wider block shortens the copy
-// loops.  Launches of G(K : x) with 256 / 128 threads, us (ncu, one GB300):
-//   passes A, E  FP64 63: 130 + 93 / 117 + 88; 27: 27 + 18 / 17 + 13; 15: 11.3 + 6.7 / 11.2 + 7.1
-//   pass B       FP64 63: 78 / 75; FP32 40: 9.6 / 8.1; 27: 5.6 / 6.9
-//   pass C       FP64 40: 48 / 38; 27: 26 / 28; FP32 48: 23 / 19; 40: 13.7 / 17.9
-int line_threads(int N) { return N >= 20 ? 128 : 256; }
-int plane_threads(int N) { return N >= 36 ? 128 : 256; }
+// Threads per block of the five-pass form's shared-memory passes (grids above small_max) and of
+// pass C, which the FP32 three-pass form runs too.  A stage has (columns x N / radix) butterflies
+// -- 81 to 162 for the radices 7 to 9 at N = 63 -- so 256 threads leave half of the block idle
+// while its registers (about 112 a thread in FP64) hold back other blocks; only pass C of small
+// FP32 grids does not fill the SMs, and there the wider block shortens the copy loops.  Launches
+// of G(K : x) with 256 / 128 threads, us (ncu, one GB300): FP64 63^3 passes A and E 130 + 93 /
+// 117 + 88, pass B 78 / 75; FP32 pass C 48^3 23 / 19, 40^3 13.7 / 17.9
+constexpr int PASS_THREADS = 128;
 template <typename T>
-int column_threads(int N) { return N >= (sizeof(T) == 8 ? 36 : 44) ? 128 : 256; }
+int column_threads(int N) { return sizeof(T) == 4 && N < 44 ? 256 : PASS_THREADS; }
 
 // ---- small grids: planes forward, columns, planes inverse (green_small.cuh) -------------
 template <typename T, bool SPLIT>
@@ -134,7 +132,7 @@ __global__ void __launch_bounds__(256) small_inverse(const typename Vec2<T>::t* 
 // half spectrum and balances better, but a plane tile reads all nine components of x for
 // each one it writes and its FP64 stages fill the lanes less well than the wider line and
 // column tiles.  Three against five passes, us per G(K : x) (ncu, one GB300): FP64 9^3 24 / 61,
-// 16^3 36 / 46, 24^3 51 / 58, 32^3 69 / 95 (register passes), 48^3 204 / 212, 56^3 367 / 331;
+// 16^3 28 / 46, 24^3 51 / 58, 32^3 69 / 95 (register passes), 48^3 204 / 212, 56^3 367 / 331;
 // FP32 15^3 21 / 31, 27^3 30 / 37, 48^3 47 / 59, 63^3 75 / 90, 80^3 174 / 193, 96^3 306 / 309.
 template <typename T>
 constexpr int small_max() { return sizeof(T) == 8 ? 48 : 80; }
@@ -221,7 +219,7 @@ cudaError_t green_apply_dot(const T* x, const T* K4, int flgK, T* y, typename Ve
     double* part_a = (g.pre && part && flgK) ? part : nullptr;
     if (part_a && nparts) *nparts = scf ? -1 : 9 * N;
     if constexpr (sizeof(T) == 8) {
-      if (N <= 16) {  // split stages: 15^3 33 against 38 us, 20^3 63 against 42
+      if (N <= 16) {  // split stages: 15^3 34 against 38 us; a call at 17^3 86 against 43, 20^3 62 against 43
         g.plan = split_plan(N);
         small_apply<T, true>(x, K4, flgK, y, S, tw, g, st, part_a, scf);
       } else {
@@ -245,14 +243,13 @@ cudaError_t green_apply_dot(const T* x, const T* K4, int flgK, T* y, typename Ve
   // operator's <x, y> is left to the caller on this path
   double* part_a = (g.pre && part && flgK) ? part : nullptr;
   if (part_a && nparts) *nparts = npair * N;
-  const int ta = line_threads(N), tb = plane_threads(N), tc = column_threads<T>(N);
-  pass_a<T, T><<<npair * N, ta, smem_a<T>(N), st>>>(x, K4, flgK, S, g, tw, part_a);
+  pass_a<T, T><<<npair * N, PASS_THREADS, smem_a<T>(N), st>>>(x, K4, flgK, S, g, tw, part_a);
   dim3 gb((H + g.tkb - 1) / g.tkb, N, 9);
-  pass_b<T><<<gb, tb, smem_b<T>(N, g.tkb), st>>>(S, g, tw, 0);
+  pass_b<T><<<gb, PASS_THREADS, smem_b<T>(N, g.tkb), st>>>(S, g, tw, 0);
   dim3 gc((H + g.tkc - 1) / g.tkc, N);
-  pass_c<T><<<gc, tc, smem_c<T>(N, g.tkc), st>>>(S, g, tw);
-  pass_b<T><<<gb, tb, smem_b<T>(N, g.tkb), st>>>(S, g, tw, 1);
-  pass_e<T><<<npair * N, ta, smem_a<T>(N), st>>>(S, y, g, tw);
+  pass_c<T><<<gc, column_threads<T>(N), smem_c<T>(N, g.tkc), st>>>(S, g, tw);
+  pass_b<T><<<gb, PASS_THREADS, smem_b<T>(N, g.tkb), st>>>(S, g, tw, 1);
+  pass_e<T><<<npair * N, PASS_THREADS, smem_a<T>(N), st>>>(S, y, g, tw);
   g_kernel_launches += 5;
   return cudaGetLastError();
 }
