@@ -131,8 +131,8 @@ __global__ void __launch_bounds__(256) small_inverse(const typename Vec2<T>::t* 
 // The largest grid of the three-pass form.  It saves two launches and one round trip of the
 // half spectrum and balances better, but a plane tile reads all nine components of x for
 // each one it writes and its FP64 stages fill the lanes less well than the wider line and
-// column tiles.  Three against five passes, us per G(K : x) (ncu, one GB300): FP64 9^3 24 / 61,
-// 16^3 28 / 46, 24^3 51 / 58, 32^3 69 / 95 (register passes), 48^3 204 / 212, 56^3 367 / 331;
+// column tiles.  Three against five passes, us per G(K : x) (ncu, one GB300): FP64 9^3 25 / 61,
+// 16^3 29 / 46, 24^3 51 / 58, 32^3 69 / 95 (register passes), 48^3 204 / 212, 56^3 367 / 331;
 // FP32 15^3 21 / 31, 27^3 30 / 37, 48^3 47 / 59, 63^3 75 / 90, 80^3 174 / 193, 96^3 306 / 309.
 template <typename T>
 constexpr int small_max() { return sizeof(T) == 8 ? 48 : 80; }
@@ -219,7 +219,7 @@ cudaError_t green_apply_dot(const T* x, const T* K4, int flgK, T* y, typename Ve
     double* part_a = (g.pre && part && flgK) ? part : nullptr;
     if (part_a && nparts) *nparts = scf ? -1 : 9 * N;
     if constexpr (sizeof(T) == 8) {
-      if (N <= 16) {  // split stages: 15^3 34 against 38 us; a call at 17^3 86 against 43, 20^3 62 against 43
+      if (N <= 16) {  // split stages: 15^3 35 against 38 us; a call at 17^3 86 against 43, 20^3 62 / 43
         g.plan = split_plan(N);
         small_apply<T, true>(x, K4, flgK, y, S, tw, g, st, part_a, scf);
       } else {

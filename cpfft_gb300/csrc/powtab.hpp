@@ -92,7 +92,9 @@ POWTAB_HD double value(int64_t b) {
 // x^y, x >= 0, with the exponent's table: x = 2^k m, the interval's 1/c from m's leading bits,
 // u = m / c - 1, w = c^y 2^(y k) with its rounding error, (1 + u)^y by its binomial series
 // (|u| <= 2^-9).  Twelve FP64 instructions where CUDA's pow takes about 95; error below 0.6 ulp
-// where x^y is a normal number and 2^-512 <= x < 2^512.  Other x (zeros of E) take pow.
+// where x^y is a normal number and 2^-512 <= x < 2^512.  Other x (zeros of E) take pow.  The FP64
+// pipe bounds the callers: a 32^3 pass of 48 systems takes 3.85 ms, without the three
+// instructions of the error terms 3.72 (up to 2.6 ulp; pow has up to 1.3).
 POWTAB_HD double tpow(const PowTab* t, double x) {
   using namespace powtab;
   const int64_t xb = bits(x);

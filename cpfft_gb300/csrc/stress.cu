@@ -12,7 +12,7 @@
 // tangent and the rotation, contractions with the trace-free Schmid tensors take five
 // products, and cep2A's 81-term loops are contracted through 3x3 intermediates (about 1.6
 // kflop instead of ~20 kflop).  One implicit pass with the reference's start on a GB300: 64^3
-// FCC Voce 22.5 to 14.7 ms, 32^3 BCC-48 (exponent 5.48) 12.4 to 3.7 ms.  Every local loop is
+// FCC Voce 22.5 to 14.7 ms, 32^3 BCC-48 (exponent 5.48) 12.4 to 3.8 ms.  Every local loop is
 // bounded by miter and the line-search cap, so no thread can spin.
 #include <algorithm>
 
