@@ -18,8 +18,9 @@ struct PowTab {
   struct alignas(16) Pair {
     double v, d;  // a value rounded to double, and what it lacks, relative to it
   };
-  Pair P[NM];     // rc^-y
-  Pair E[NE];     // 2^(y (k - EMID)); zero where x^y isn't normal on all of [2^k, 2^(k + 1)]
+  Pair P[NM];      // rc^-y
+  // 2^(y (k - EMID)); zero where x^y isn't normal on all of that binade, and at NE (other binades)
+  Pair E[NE + 1];
   double rc[NM];  // 1 / c, rounded
   double c[6];    // binomial coefficients y, y (y - 1) / 2, .. of (1 + u)^y - 1
   double y;
@@ -45,6 +46,7 @@ inline bool pow_table(double y, PowTab& t) {
     t.rc[i] = (double)(1.0L / (1.0L + (i + 0.5L) / PowTab::NM));
     t.P[i] = powtab::pair(powl((long double)t.rc[i], -(long double)y));
   }
+  t.E[PowTab::NE] = {0.0, 0.0};
   for (int k = 0; k < PowTab::NE; k++) {
     const int e = k - PowTab::EMID;
     const bool normal = y * e >= -1022.0 && y * (e + 1) <= 1023.0;
@@ -69,20 +71,24 @@ POWTAB_HD PowTab::Pair load(const PowTab::Pair* p) {
   return *p;
 #endif
 }
-POWTAB_HD int64_t bits(double x) {
+// a double's words (the device's own 32-bit forms: through 64-bit masks the stress kernels spill
+// more, 0.7 % of a fast-form pass at 128^3)
+POWTAB_HD int high(double x) {
 #ifdef __CUDA_ARCH__
-  return __double_as_longlong(x);
+  return __double2hiint(x);
 #else
   int64_t b;
   std::memcpy(&b, &x, 8);
-  return b;
+  return (int)(b >> 32);
 #endif
 }
-POWTAB_HD double value(int64_t b) {
+POWTAB_HD double with_high(double x, int hi) {
 #ifdef __CUDA_ARCH__
-  return __longlong_as_double(b);
+  return __hiloint2double(hi, __double2loint(x));
 #else
-  double x;
+  int64_t b;
+  std::memcpy(&b, &x, 8);
+  b = (int64_t)((uint64_t)(uint32_t)hi << 32) | (b & 0xffffffff);
   std::memcpy(&x, &b, 8);
   return x;
 #endif
@@ -97,14 +103,13 @@ POWTAB_HD double value(int64_t b) {
 // instructions of the error terms 3.72 (up to 2.6 ulp; pow has up to 1.3).
 POWTAB_HD double tpow(const PowTab* t, double x) {
   using namespace powtab;
-  const int64_t xb = bits(x);
-  const int hi = (int)(xb >> 32);
+  const int hi = high(x);
   const unsigned k = (unsigned)((hi >> 20) - 1023 + PowTab::EMID);
-  const PowTab::Pair e = k < PowTab::NE ? load(t->E + k) : PowTab::Pair{0.0, 0.0};
-  if (bits(e.v) == 0) return x == 0.0 ? 0.0 : pow(x, t->y);
+  const PowTab::Pair e = load(t->E + (k < PowTab::NE ? k : PowTab::NE));
+  if (high(e.v) == 0) return x == 0.0 ? 0.0 : pow(x, t->y);
   const int i = (hi >> 12) & (PowTab::NM - 1);
   const PowTab::Pair p = load(t->P + i);
-  const double m = value((xb & 0xfffffffffffffLL) | 0x3ff0000000000000LL);
+  const double m = with_high(x, (hi & 0xfffff) | 0x3ff00000);
   const double u = fma(m, load(t->rc + i), -1.0);
   const double w = p.v * e.v, dw = fma(p.v, e.v, -w);
   double q = load(t->c + 5);
